@@ -1,77 +1,287 @@
 // True float32 matrix product for the 32-bit path of the model:
 //   C[M, N] = A[M, K] * W[N, K]^T      (the layout of a Linear weight: y = x W^T)
-// Plain FFMA on CUDA cores: no tensor cores, no TF32, no split-K.  Every output
-// element is the sum over k = 0..K-1 in ascending order, tile of 16 by tile of 16,
-// so a row's result does not depend on M or on the rest of the batch.
-// This is the slow, checkable path; the serving path uses tensor cores.
+// FFMA on CUDA cores: no tensor cores, no TF32.
+//
+// The order of an output's additions depends on k alone, so a row's result does not depend on M, on the rest of the
+// batch or on which of the two kernels below computes it.  With k = 1024 s + 256 j + 8 l + i (j < 4, l < 32, i < 8):
+//   chain(s, l) = the FMA chain over j, then i, ascending, from zero            (32 terms)
+//   T_g         = the chains of l = 8 g .. 8 g + 7, s by s, l ascending, added one after the other (g < 4)
+//   C           = (T_0 + T_1) + (T_2 + T_3)
+// It is made for both kernels: l is the lane that streams a weight row in pieces of 32 bytes where few rows of A make
+// the product a stream over W, and g is one of four groups of threads that share the K of an output tile.  Short chains,
+// summed by groups, are also closer to 64 bits than one sum over K in tiles of 16, which was the order before (of the result's
+// norm, normal values: 1.24e-7 against 1.60e-7 at K = 1,024, 1.44e-7 against 2.56e-7 at K = 3,072).
 #include "common.cuh"
 
 namespace q3 {
 
-constexpr int GF_BM = 64, GF_BN = 64, GF_BK = 16, GF_THREADS = 256;
+constexpr int GF_SEG = 1024;  // values of k in a segment s
+constexpr int GF_STEP = 256;  // from one j to the next
+constexpr int GF_LANE = 8;    // values of k of a lane at a time
 
-__global__ void __launch_bounds__(GF_THREADS)
-gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
-                   int M, int N, int K, int lda, int ldw, int ldc) {
+// ---------------------------------------------------------------- tiles
+// 64 x 64 outputs per block, four groups of 64 threads; group g walks over its chains (s, l) with 8 x 8 outputs per thread
+// and the four partial sums meet in shared memory.  Bound by the FMA pipe: 64 FMA per four 16-byte shared-memory reads.
+// The split over K inside the block gives a narrow product (N = 1,024 and 500 rows: 144 tiles of 64 x 64) a block on
+// every SM with eight warps of 8 x 8 register tiles, which tiles of 128 x 128 (32 blocks) could not.
+constexpr int GF_T = 64, GF_GROUPS = 4, GF_GROUP_THREADS = 64, GF_THREADS = GF_GROUPS * GF_GROUP_THREADS, GF_STAGES = 3;
+constexpr int GF_STAGE_BYTES = 2 * GF_T * 128;                            // 64 rows of A, 64 of W, 32 values of k each
+constexpr int GF_RED_PITCH = GF_T + 8;                                    // floats: a thread's rows fall on different banks
+constexpr int GF_SMEM = GF_GROUPS * GF_STAGES * GF_STAGE_BYTES;           // 192 KB; the partial sums reuse it
+static_assert(GF_GROUPS * GF_T * GF_RED_PITCH * 4 <= GF_SMEM, "the partial sums fit");
+
+template <int BYTES>
+__device__ __forceinline__ void gf_copy(uint32_t dst, const float* src, bool in) {
+  const int n = in ? BYTES : 0;  // zero bytes read: the destination is filled with zeros
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ float4 gf_lds(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+
+// VEC: K, lda, ldw are multiples of 4 and A, W are 16-byte aligned (copies of 16 bytes; otherwise of 4).
+template <bool VEC>
+__global__ void __launch_bounds__(GF_THREADS, 1)
+gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
+                     int lda, int ldw, int ldc, int out_vec) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float As[GF_BK][GF_BM + 4];
-  __shared__ float Ws[GF_BK][GF_BN + 4];
-  const int m0 = blockIdx.y * GF_BM, n0 = blockIdx.x * GF_BN;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  extern __shared__ __align__(1024) unsigned char gf_smem[];
+  const int group = threadIdx.x / GF_GROUP_THREADS, t = threadIdx.x % GF_GROUP_THREADS;
+  const int m_tiles = (M + GF_T - 1) / GF_T;  // tiles of the same W rows next to each other: a wave of blocks reads W once
+  const int m0 = (blockIdx.x % m_tiles) * GF_T, n0 = (blockIdx.x / m_tiles) * GF_T;
+  const uint32_t stages = (uint32_t)__cvta_generic_to_shared(gf_smem) + group * GF_STAGES * GF_STAGE_BYTES;
 
-  // each thread stages 4 elements of each tile: tile row = e / BK, tile col = e % BK
-  for (int k0 = 0; k0 < K; k0 += GF_BK) {
+  // a stage: row r's 32 values of chain (s, l) as eight pieces of 16 bytes (piece c: j = c / 2, half c % 2), piece c at
+  // place c ^ (r % 8), so that eight rows' equal pieces lie on different banks
+  const int c = t & 7, r8 = t >> 3;
+  const int k_piece = (c >> 1) * GF_STEP + (c & 1) * 4;
+  const uint32_t dst0 = r8 * 128 + ((c ^ r8) << 4);
+  const int segs = (K + GF_SEG - 1) / GF_SEG, items = segs * 8;
+  auto fetch = [&](int item) {
+    const int k = (item >> 3) * GF_SEG + k_piece + (group * 8 + (item & 7)) * GF_LANE;
+    const uint32_t dst = stages + (item % GF_STAGES) * GF_STAGE_BYTES + dst0;
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const int e = threadIdx.x + p * GF_THREADS;
-      const int r = e / GF_BK, c = e % GF_BK;
-      const int k = k0 + c;
-      const int am = m0 + r, wn = n0 + r;
-      As[c][r] = (am < M && k < K) ? A[(size_t)am * lda + k] : 0.f;
-      Ws[c][r] = (wn < N && k < K) ? W[(size_t)wn * ldw + k] : 0.f;
+    for (int p = 0; p < 16; ++p) {
+      const int r = r8 + 8 * (p & 7), row = (p < 8 ? m0 : n0) + r, rows = p < 8 ? M : N;
+      const float* src = (p < 8 ? A + (size_t)min(row, M - 1) * lda : W + (size_t)min(row, N - 1) * ldw);
+      if (VEC) {
+        const bool in = row < rows && k < K;
+        gf_copy<16>(dst + p * 1024, src + (in ? k : 0), in);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool in = row < rows && k + e < K;
+          gf_copy<4>(dst + p * 1024 + 4 * e, src + (in ? k + e : 0), in);
+        }
+      }
     }
-    __syncthreads();
-    // the 16 products of a tile are summed on their own and the tile's sum is added to the total: the rounding
-    // error of a long reduction then grows with the number of tiles, not of terms (the order still depends on k alone)
-    float part[4][4];
+  };
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < GF_STAGES - 1; ++i) {
+    if (i < items) fetch(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+
+  const int tx = t & 7, ty = t >> 3;  // rows ty + 8 i of A, tx + 8 j of W
+  float total[8][8], part[8][8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int kk = 0; kk < GF_BK; ++kk) {
-      float a[4], b[4];
+    for (int j = 0; j < 8; ++j) total[i][j] = 0.f;
+
+  for (int item = 0; item < items; ++item) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GF_STAGES - 2) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(GF_GROUP_THREADS) : "memory");  // the group's copies are there,
+    if (item + GF_STAGES - 1 < items) fetch(item + GF_STAGES - 1);  // and the stage read in the last turn is free
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const uint32_t base = stages + (item % GF_STAGES) * GF_STAGE_BYTES;
+    const uint32_t a_row = base + ty * 128, w_row = base + GF_T * 128 + tx * 128;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Ws[kk][tx * 4 + j];
+      for (int j = 0; j < 8; ++j) part[i][j] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      float4 a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = gf_lds(a_row + i * 1024 + ((q ^ ty) << 4));
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 w = gf_lds(w_row + j * 1024 + ((q ^ tx) << 4));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].x, w.x, part[i][j]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].y, w.y, part[i][j]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].z, w.z, part[i][j]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].w, w.w, part[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) total[i][j] += part[i][j];
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float* red = reinterpret_cast<float*>(gf_smem);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[(group * GF_T + ty + 8 * i) * GF_RED_PITCH + tx + 8 * j] = total[i][j];
+  __syncthreads();
+  // four neighbouring outputs per thread and turn
+  for (int e = threadIdx.x; e < GF_T * GF_T / 4; e += GF_THREADS) {
+    const int r = e / (GF_T / 4), col = (e % (GF_T / 4)) * 4;
+    if (m0 + r >= M || n0 + col >= N) continue;
+    float4 T[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) T[g] = *reinterpret_cast<const float4*>(&red[(g * GF_T + r) * GF_RED_PITCH + col]);
+    const float v[4] = {(T[0].x + T[1].x) + (T[2].x + T[3].x), (T[0].y + T[1].y) + (T[2].y + T[3].y),
+                        (T[0].z + T[1].z) + (T[2].z + T[3].z), (T[0].w + T[1].w) + (T[2].w + T[3].w)};
+    float* dst = C + (size_t)(m0 + r) * ldc + n0 + col;
+    if (out_vec && n0 + col + 4 <= N) {
+      *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) part[i][j] = fmaf(a[i], b[j], part[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+        if (n0 + col + i < N) dst[i] = v[i];
     }
   }
+}
+
+// ---------------------------------------------------------------- a few rows of A
+// Decoding: the product is one pass over W, so the weights go from memory straight into the registers that multiply them,
+// 32 bytes per lane and load, and each warp takes R weight rows over one segment of 1,024 values of k (8 KB of loads in
+// flight per warp with R = 4; the first of them before the wait on the kernel before, which never writes weights).  The
+// rows of A come through L1, which the block's warps share.  The chains' sums meet in shared memory.
+constexpr int GFS_WARPS = 8;
+constexpr int GFS_MAX_ROWS = 16;
+
+__device__ __forceinline__ void gf_load8(float (&v)[8], const float* p) {  // read once: not kept in L1
+  asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(p));
+}
+__device__ __forceinline__ void gf_load8_shared(float (&v)[8], const float* p) {  // the block's warps all read it
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(p));
+}
+
+// MT: rows of A (M <= MT; those past M repeat the last one and are not stored).  seg_warps: warps of the block that share
+// a group of R weight rows, each with every seg_warps-th segment.  K, lda, ldw multiples of 8, A and W 32-byte aligned.
+template <int MT, int R>
+__global__ void __launch_bounds__(GFS_WARPS * 32, MT <= 8 ? 2 : 1)
+gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
+                     int lda, int ldw, int ldc, int seg_warps) {
+  extern __shared__ __align__(16) float gfs_sums[];  // [output of the block][segment][lane]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int segs = (K + GF_SEG - 1) / GF_SEG;
+  const int groups = GFS_WARPS / seg_warps;  // of weight rows per block
+  const int group = warp / seg_warps, first = warp % seg_warps;
+  const int n0 = (blockIdx.x * groups + group) * R;
+  const bool active = group < groups && n0 < N && first < segs;
+
+  const float* w_row[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) w_row[r] = W + (size_t)min(n0 + r, N - 1) * ldw + lane * GF_LANE;
+  float w[2][R][8];
+  auto load_w = [&](float (&dst)[R][8], int s, int j) {
+    const int k = s * GF_SEG + j * GF_STEP;
+    const bool in = s < segs && k + lane * GF_LANE < K;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (in) {
+        gf_load8(dst[r], w_row[r] + k);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dst[r][i] = 0.f;
+      }
+    }
+  };
+  if (active) {
+    load_w(w[0], first, 0);
+    load_w(w[1], first, 1);
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (active) {
+    for (int s = first; s < segs; s += seg_warps) {
+      float acc[R][MT];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int k = s * GF_SEG + j * GF_STEP + lane * GF_LANE;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          float x[8];
+          if (k < K) {
+            gf_load8_shared(x, A + (size_t)min(m, M - 1) * lda + k);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = 0.f;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[r][m] = fmaf(x[i], w[j & 1][r][i], acc[r][m]);
+        }
+        if (j < 2) load_w(w[j & 1], s, j + 2);
+        else load_w(w[j & 1], s + seg_warps, j - 2);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+          gfs_sums[((size_t)((group * R + r) * MT + m) * segs + s) * 32 + lane] = acc[r][m];
+    }
+  }
+  __syncthreads();
+  // four threads per output: T_g of the head of the file, then their sums
+  const int outputs = groups * R * MT;
+  for (int e0 = 0; e0 < outputs * 4; e0 += GFS_WARPS * 32) {  // whole warps: the shuffles below
+    const int e = e0 + threadIdx.x, o = e >> 2, g = e & 3;
+    const int m = o % MT, n = (blockIdx.x * groups) * R + o / MT;
+    const bool live = o < outputs && m < M && n < N;
+    float T = 0.f;
+    if (live) {
+      const float* p = gfs_sums + (size_t)o * segs * 32 + g * 8;
+      for (int s = 0; s < segs; ++s) {
+        const float4 a = *reinterpret_cast<const float4*>(p + s * 32), b = *reinterpret_cast<const float4*>(p + s * 32 + 4);
+        T += a.x; T += a.y; T += a.z; T += a.w;
+        T += b.x; T += b.y; T += b.z; T += b.w;
+      }
+    }
+    T += __shfl_xor_sync(0xffffffffu, T, 1);
+    T += __shfl_xor_sync(0xffffffffu, T, 2);
+    if (live && g == 0) C[(size_t)m * ldc + n] = T;
+  }
+}
+
+template <int MT, int R>
+static int gemm_f32_rows_launch(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                                int segs, int seg_warps, cudaStream_t stream) {
+  const int groups = GFS_WARPS / seg_warps;
+  const size_t smem = (size_t)groups * R * MT * segs * 32 * sizeof(float);
+  auto kernel = gemm_f32_rows_kernel<MT, R>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  q3::launch(kernel, dim3((N + groups * R - 1) / (groups * R)), dim3(GFS_WARPS * 32), smem, stream, A, W, C, M, N, K, lda, ldw,
+             ldc, seg_warps);
+  return launch_status();
 }
 
 }  // namespace q3
@@ -79,10 +289,34 @@ gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
 // C[M, N] = A[M, K] * W[N, K]^T, all float32, row pitches lda / ldw / ldc in elements.
 extern "C" int q3_gemm_f32_nt(const float* A, const float* W, float* C, int M, int N, int K, int lda,
                               int ldw, int ldc, cudaStream_t stream) {
+  using namespace q3;
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return Q3_ERR_SIZE;
-  dim3 grid((N + q3::GF_BN - 1) / q3::GF_BN, (M + q3::GF_BM - 1) / q3::GF_BM);
-  if (grid.y > 65535) return Q3_ERR_SIZE;
-  q3::launch(q3::gemm_f32_nt_kernel, dim3(grid), dim3(q3::GF_THREADS), 0, stream, A, W, C, M, N, K, lda, ldw, ldc);
-  return q3::launch_status();
+  const int segs = (K + GF_SEG - 1) / GF_SEG;
+  // Up to 16 rows stream W once; the sums of up to 16 segments (K = 16,384) fit the block's shared memory.
+  if (M <= GFS_MAX_ROWS && segs <= 16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && (uintptr_t)A % 32 == 0 &&
+      (uintptr_t)W % 32 == 0) {
+    const int seg_warps = segs < GFS_WARPS ? segs : GFS_WARPS;
+    const int groups = GFS_WARPS / seg_warps;
+    // four weight rows per warp share the reads of A; two where four would leave SMs without a block
+    const bool four = (N + groups * 4 - 1) / (groups * 4) >= sm_count() * 3 / 4;
+#define Q3_GFS_GO(MT)                                                                                              \
+  return four ? gemm_f32_rows_launch<MT, 4>(A, W, C, M, N, K, lda, ldw, ldc, segs, seg_warps, stream)              \
+              : gemm_f32_rows_launch<MT, 2>(A, W, C, M, N, K, lda, ldw, ldc, segs, seg_warps, stream)
+    if (M == 1) Q3_GFS_GO(1);
+    if (M == 2) Q3_GFS_GO(2);
+    if (M <= 4) Q3_GFS_GO(4);
+    if (M <= 8) Q3_GFS_GO(8);
+    Q3_GFS_GO(16);
+#undef Q3_GFS_GO
+  }
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+  const int out_vec = ldc % 4 == 0 && (uintptr_t)C % 16 == 0;
+  const long long m_tiles = (M + GF_T - 1) / GF_T, n_tiles = (N + GF_T - 1) / GF_T;
+  if (m_tiles > 65535 || m_tiles * n_tiles > 0x7fffffffll) return Q3_ERR_SIZE;
+  auto kernel = vec ? gemm_f32_tile_kernel<true> : gemm_f32_tile_kernel<false>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
+  if (e != cudaSuccess) return (int)e;
+  q3::launch(kernel, dim3((unsigned)(m_tiles * n_tiles)), dim3(GF_THREADS), GF_SMEM, stream, A, W, C, M, N, K, lda, ldw, ldc, out_vec);
+  return launch_status();
 }

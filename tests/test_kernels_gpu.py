@@ -167,6 +167,24 @@ def test_gemm_f32_is_true_float32(shape):
     assert torch.equal(one[0], out[M // 2])
 
 
+@pytest.mark.parametrize("N,K", [(70, 8), (133, 248), (1000, 1024), (64, 1032), (4096, 1024), (517, 3072), (1024, 2056),
+                                 (40, 9000)])
+def test_gemm_f32_orders_agree(N, K):
+    """The kernel for a few rows (K a multiple of 8) and the tiles give the same bits for every row: the order of the
+    additions is a function of k.  Rows at the edges of both kernels' tiles; the weights' row pitch is K."""
+    g = torch.Generator().manual_seed(5)
+    a, w = torch.randn(67, K, generator=g), torch.randn(N, K, generator=g)
+    A, W = dev(a), dev(w)
+    out = torch.empty(67, N, device="cuda")
+    ops().gemm_f32_nt(A, W, out)  # two tiles of rows
+    want = a.double() @ w.double().t()
+    assert float((out.cpu().double() - want).abs().max()) <= 1e-6 * K ** 0.5 * float(want.abs().max())
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 64, 65):
+        wide = torch.full((M, N + 3), float("nan"), device="cuda")  # into columns of a wider buffer
+        ops().gemm_f32_nt(A[:M].contiguous(), W, wide[:, :N])
+        assert torch.equal(wide[:, :N], out[:M]) and bool(torch.isnan(wide[:, N:]).all()), M
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 def test_swiglu(dtype):
     g = torch.Generator().manual_seed(4)
