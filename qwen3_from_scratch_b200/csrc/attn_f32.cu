@@ -1,0 +1,356 @@
+// Paged causal attention in float32 for head sizes 64 and 128: the 32-bit path's attention (scores, probabilities and
+// sums in float32, on CUDA cores), for whole prompts, portions and single tokens.
+//
+// A query's result depends only on its own keys, not on how the batch was cut or on the kernel that computes it.  The keys
+// are taken in chunks of 64 by their absolute position, and for each chunk that holds a key the query sees:
+//   s_n = scale * (q . k_n)        the dot product by runs of 16 values, the runs added one after the other
+//   m_c = max s_n,  p_n = exp(s_n - m_c),  l_c = sum p_n (keys t, t + 16, t + 32, t + 48 first, then over t by halves)
+//   o_c = sum p_n v_n              ascending n
+// and the chunks are folded together in ascending order: m' = max(m, m_c), l' = l exp(m - m') + l_c exp(m_c - m'), o likewise.
+// Long contexts keep their accuracy (sums of 64, then one term per chunk), and the chunks of a single token can be
+// computed side by side:
+//   attn_f32_kernel, whole      a block takes 16 or 32 (token, head) rows of one kv head and walks over the chunks
+//   attn_f32_kernel, by chunks  a block takes the heads of one token and one chunk and leaves (m_c, l_c, o_c)
+//   attn_f32_fold_kernel        folds them
+// Sizes of the 0.6B model (16 heads over 8 of 128), cold caches: 4 single tokens at contexts of 400 to 900 31.7 us, one at
+// 4,096 69 us, prompts of 203 and 310 tokens 76 us; the walk over the keys one by one that served here before (attn_ref.cu,
+// a warp per token and head) took 1,435, 6,600 and 453 us: some 1.6 us per key of the longest context, whatever the batch.
+//
+// Reference formulas: as in attn_ref.cu (models/attn.py:402-499, kernels/triton/paged_attn.py:89-181).
+#include "common.cuh"
+
+namespace q3 {
+
+constexpr int AF_THREADS = 128, AF_CHUNK = 64;
+constexpr float AF_MASKED = -1.0f;  // in place of a probability: the query does not see the key
+
+__device__ __forceinline__ void af_copy16(uint32_t dst, const float* src, bool in) {
+  const int n = in ? 16 : 0;  // zero bytes read: the destination is filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ float4 af_lds(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// RPT: rows per thread; the block has 8 RPT (token, head) rows of one kv head, row r = token r / G, head r % G of the group.
+template <int D, int RPT>
+struct AfShape {
+  static constexpr int ROWS = 8 * RPT;
+  static constexpr size_t SMEM = ((size_t)(ROWS + 2 * AF_CHUNK) * D + (size_t)ROWS * AF_CHUNK) * sizeof(float);
+};
+
+// BY_CHUNK: grid (chunks, kv heads, requests), single-token requests only; else grid (token tiles, kv heads, requests).
+// Bound by shared-memory reads and the FMA pipe together (a 4 x 4 piece of the scores per thread: 8 reads of 16 bytes for
+// 64 FMA); K of the next chunk is fetched under P V, V under the scores.
+template <int D, int RPT, bool BY_CHUNK>
+__global__ void __launch_bounds__(AF_THREADS)
+attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                float* __restrict__ out, float* __restrict__ partial, const int* __restrict__ q_start,
+                const int* __restrict__ kv_len, const int* __restrict__ block_table, int table_stride, int page_size,
+                int num_pages, int Hq, int Hkv, float scale, int window, int max_chunks, int* status) {
+  constexpr int ROWS = 8 * RPT, D4 = D / 4, DV = D / 64;  // DV: pieces of four output columns per thread
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(128) float af_smem[];
+  float* q_s = af_smem;                  // [ROWS][D], piece c of a row at place c ^ (row & 7)
+  float* k_s = q_s + ROWS * D;           // [64][D], the same
+  float* v_s = k_s + AF_CHUNK * D;       // [64][D], as it is
+  float* p_s = v_s + AF_CHUNK * D;       // [ROWS][64], as Q
+  __shared__ unsigned long long key_ok;  // bit n: key n of the chunk has a page
+
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;  // rows ty + 8 i, keys tx + 16 j
+  const int b = blockIdx.z, hk = blockIdx.y, G = Hq / Hkv;
+  const int t0 = q_start[b], q_len = q_start[b + 1] - t0, len = kv_len[b];
+  const int tokens = ROWS / G, tok0 = BY_CHUNK ? 0 : blockIdx.x * tokens;
+  if (tok0 >= q_len) return;
+  const int live_rows = min(tokens, q_len - tok0) * G;
+  const int first_pos = len - q_len + tok0, last_pos = first_pos + min(tokens, q_len - tok0) - 1;
+  const int first_key = (window > 0 && first_pos - window + 1 > 0) ? first_pos - window + 1 : 0;
+  int chunk = BY_CHUNK ? blockIdx.x : first_key / AF_CHUNK;
+  const int chunk_end = BY_CHUNK ? chunk + 1 : last_pos / AF_CHUNK + 1;
+  if (first_pos < 0 && tid == 0 && (!BY_CHUNK || chunk == 0)) atomicOr(status, Q3_STATUS_BAD_POSITION);
+  if (BY_CHUNK && (chunk * AF_CHUNK > last_pos || (chunk + 1) * AF_CHUNK <= first_key)) return;
+
+  for (int e = tid; e < ROWS * D4; e += AF_THREADS) {
+    const int r = e / D4, c = e % D4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < live_rows) v = af_lds(q + ((size_t)(t0 + tok0 + r / G) * Hq + hk * G + r % G) * D + c * 4);
+    *reinterpret_cast<float4*>(q_s + r * D + ((c ^ (r & 7)) * 4)) = v;
+  }
+  int pos[RPT], lo[RPT];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = ty + 8 * i;
+    pos[i] = r < live_rows ? first_pos + r / G : -1;
+    lo[i] = (window > 0 && pos[i] - window + 1 > 0) ? pos[i] - window + 1 : 0;
+  }
+  const bool busy = (tid >> 5) * 2 < live_rows;  // the warp's first row is in use (its rows: 2 w, 2 w + 1, then by 8)
+
+  const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(k_s), v_addr = (uint32_t)__cvta_generic_to_shared(v_s);
+  const int* table = block_table + (size_t)b * table_stride;
+  // two threads per key: its page, then its row piece by piece
+  const int my_key = tid >> 1;
+  auto fetch = [&](uint32_t dst, const float* pages, int c, bool swizzle, bool note) {
+    const int n = c * AF_CHUNK + my_key;
+    int page = -1;
+    if (n >= first_key && n <= last_pos) {
+      page = table_page(table, n / page_size, table_stride, status);
+      if (page < 0 || page >= num_pages) {
+        if (note) atomicOr(status, Q3_STATUS_BAD_PAGE);
+        page = -1;
+      }
+    }
+    const float* src = pages + (page < 0 ? 0 : (((size_t)page * Hkv + hk) * page_size + n % page_size) * D);
+#pragma unroll
+    for (int i = 0; i < D4 / 2; ++i) {
+      const int piece = 2 * i + (tid & 1);
+      af_copy16(dst + (my_key * D + (swizzle ? piece ^ (my_key & 7) : piece) * 4) * 4, src + piece * 4, page >= 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    return page >= 0;
+  };
+
+  float m[RPT], l[RPT], o[RPT][4 * DV];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int d = 0; d < 4 * DV; ++d) o[i][d] = 0.f;
+  }
+  bool have = false;
+  if (chunk < chunk_end) have = fetch(k_addr, k_pages, chunk, true, true);
+  for (; chunk < chunk_end; ++chunk) {
+    if (tid == 0) key_ok = 0ull;
+    __syncthreads();  // V and P of the chunk before have been read
+    if (!(tid & 1) && have) atomicOr(&key_ok, 1ull << my_key);
+    fetch(v_addr, v_pages, chunk, false, false);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // K and key_ok (and Q)
+    const unsigned long long ok = key_ok;
+    float oc[RPT][4 * DV], mc[RPT], lc[RPT];
+    if (busy) {
+      float s[RPT][4];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 1
+      for (int run = 0; run < D / 16; ++run) {
+        float part[RPT][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float4 kv[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) kv[j] = af_lds(k_s + (tx + 16 * j) * D + (((run * 4 + c) ^ (tx & 7)) * 4));
+#pragma unroll
+          for (int i = 0; i < RPT; ++i) {
+            const float4 a = af_lds(q_s + (ty + 8 * i) * D + (((run * 4 + c) ^ ty) * 4));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              part[i][j] = c == 0 ? a.x * kv[j].x : fmaf(a.x, kv[j].x, part[i][j]);
+              part[i][j] = fmaf(a.y, kv[j].y, part[i][j]);
+              part[i][j] = fmaf(a.z, kv[j].z, part[i][j]);
+              part[i][j] = fmaf(a.w, kv[j].w, part[i][j]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[i][j] += part[i][j];
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        bool sees[4];
+        mc[i] = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = tx + 16 * j, n = chunk * AF_CHUNK + key;
+          sees[j] = n >= lo[i] && n <= pos[i] && ((ok >> key) & 1ull);
+          s[i][j] *= scale;
+          if (sees[j]) mc[i] = fmaxf(mc[i], s[i][j]);
+        }
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) mc[i] = fmaxf(mc[i], __shfl_xor_sync(0xffffffffu, mc[i], x));
+        lc[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float p = sees[j] ? expf(s[i][j] - mc[i]) : AF_MASKED;
+          if (sees[j]) lc[i] += p;
+          p_s[(ty + 8 * i) * AF_CHUNK + (((tx >> 2) + 4 * j) ^ ty) * 4 + (tx & 3)] = p;
+        }
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) lc[i] += __shfl_xor_sync(0xffffffffu, lc[i], x);
+      }
+    }
+    __syncthreads();  // K has been read
+    have = false;
+    if (chunk + 1 < chunk_end) have = fetch(k_addr, k_pages, chunk + 1, true, true);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // V
+    if (!busy) continue;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+#pragma unroll
+      for (int d = 0; d < 4 * DV; ++d) oc[i][d] = 0.f;
+#pragma unroll 1
+    for (int n4 = 0; n4 < AF_CHUNK; n4 += 4) {
+      float4 p4[RPT];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) p4[i] = af_lds(p_s + (ty + 8 * i) * AF_CHUNK + ((n4 >> 2) ^ ty) * 4);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        float4 v[DV];
+#pragma unroll
+        for (int c = 0; c < DV; ++c) v[c] = af_lds(v_s + (n4 + n) * D + (tx + 16 * c) * 4);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const float p = n == 0 ? p4[i].x : n == 1 ? p4[i].y : n == 2 ? p4[i].z : p4[i].w;
+          if (!(p < 0.f)) {  // a key that the query does not see takes no part, whatever its value holds
+#pragma unroll
+            for (int c = 0; c < DV; ++c) {
+              oc[i][4 * c] = fmaf(p, v[c].x, oc[i][4 * c]);
+              oc[i][4 * c + 1] = fmaf(p, v[c].y, oc[i][4 * c + 1]);
+              oc[i][4 * c + 2] = fmaf(p, v[c].z, oc[i][4 * c + 2]);
+              oc[i][4 * c + 3] = fmaf(p, v[c].w, oc[i][4 * c + 3]);
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = ty + 8 * i;
+      if constexpr (BY_CHUNK) {
+        if (r >= live_rows) continue;
+        float* dst = partial + ((size_t)(b * Hq + hk * G + r) * max_chunks + chunk) * (D + 4);
+#pragma unroll
+        for (int c = 0; c < DV; ++c)
+          *reinterpret_cast<float4*>(dst + (tx + 16 * c) * 4) =
+              make_float4(oc[i][4 * c], oc[i][4 * c + 1], oc[i][4 * c + 2], oc[i][4 * c + 3]);
+        if (tx == 0) *reinterpret_cast<float4*>(dst + D) = make_float4(mc[i], lc[i], 0.f, 0.f);
+      } else if (!(mc[i] == -INFINITY && lc[i] == 0.f)) {  // else: no key of the chunk is seen
+        const float mn = fmaxf(m[i], mc[i]), f = expf(m[i] - mn), g = expf(mc[i] - mn);
+        l[i] = fmaf(l[i], f, lc[i] * g);
+#pragma unroll
+        for (int d = 0; d < 4 * DV; ++d) o[i][d] = fmaf(o[i][d], f, oc[i][d] * g);
+        m[i] = mn;
+      }
+    }
+  }
+  if constexpr (!BY_CHUNK) {
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = ty + 8 * i;
+      if (r >= live_rows) continue;
+      const float inv = l[i] == 0.f ? 0.f : 1.0f / l[i];
+      float* dst = out + ((size_t)(t0 + tok0 + r / G) * Hq + hk * G + r % G) * D;
+#pragma unroll
+      for (int c = 0; c < DV; ++c)
+        *reinterpret_cast<float4*>(dst + (tx + 16 * c) * 4) =
+            make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+    }
+  }
+}
+
+// One block per (request, head), a thread per output value.
+template <int D>
+__global__ void __launch_bounds__(D)
+attn_f32_fold_kernel(const float* __restrict__ partial, float* __restrict__ out, const int* __restrict__ q_start,
+                     const int* __restrict__ kv_len, int Hq, int window, int max_chunks, int* status) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int b = blockIdx.y, head = blockIdx.x, d = threadIdx.x;
+  const int t = q_start[b], pos = kv_len[b] - 1;
+  if (q_start[b + 1] == t) return;
+  const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  const float* src = partial + (size_t)(b * Hq + head) * max_chunks * (D + 4);
+  float m = -INFINITY, l = 0.f, o = 0.f;
+  const int end = min(pos / AF_CHUNK + 1, max_chunks);
+  if (pos >= 0 && pos / AF_CHUNK >= max_chunks && d == 0) atomicOr(status, Q3_STATUS_BAD_POSITION);
+  if (pos >= 0) {
+#pragma unroll 4
+    for (int c = lo / AF_CHUNK; c < end; ++c) {
+      const float* p = src + (size_t)c * (D + 4);
+      const float oc = p[d], mc = p[D], lc = p[D + 1];
+      if (mc == -INFINITY && lc == 0.f) continue;
+      const float mn = fmaxf(m, mc), f = expf(m - mn), g = expf(mc - mn);
+      l = fmaf(l, f, lc * g);
+      o = fmaf(o, f, oc * g);
+      m = mn;
+    }
+  }
+  out[((size_t)t * Hq + head) * D + d] = l == 0.f ? 0.f : o * (1.0f / l);
+}
+
+template <int D, int RPT, bool BY_CHUNK>
+static int attn_f32_launch(dim3 grid, const float* q, const float* k_pages, const float* v_pages, float* out, float* partial,
+                           const int* q_start, const int* kv_len, const int* block_table, int table_stride, int page_size,
+                           int num_pages, int Hq, int Hkv, float scale, int window, int max_chunks, int* status,
+                           cudaStream_t stream) {
+  constexpr size_t smem = AfShape<D, RPT>::SMEM;
+  auto kernel = attn_f32_kernel<D, RPT, BY_CHUNK>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  q3::launch(kernel, grid, dim3(AF_THREADS), smem, stream, q, k_pages, v_pages, out, partial, q_start, kv_len, block_table,
+             table_stride, page_size, num_pages, Hq, Hkv, scale, window, max_chunks, status);
+  return launch_status();
+}
+
+template <int D>
+static int attn_f32_go(const float* q, const float* k_pages, const float* v_pages, float* out, float* partial,
+                       const int* q_start, const int* kv_len, const int* block_table, int table_stride, int page_size,
+                       int num_pages, int num_seqs, int max_q_len, int Hq, int Hkv, float scale, int window, int max_chunks,
+                       int* status, cudaStream_t stream) {
+  const int G = Hq / Hkv;
+  if (max_chunks > 0) {
+    const int code = attn_f32_launch<D, 1, true>(dim3(max_chunks, Hkv, num_seqs), q, k_pages, v_pages, out, partial, q_start,
+                                                 kv_len, block_table, table_stride, page_size, num_pages, Hq, Hkv, scale,
+                                                 window, max_chunks, status, stream);
+    if (code) return code;
+    q3::launch(attn_f32_fold_kernel<D>, dim3(Hq, num_seqs), dim3(D), 0, stream, partial, out, q_start, kv_len, Hq, window,
+               max_chunks, status);
+    return launch_status();
+  }
+  if (max_q_len * G <= 8)
+    return attn_f32_launch<D, 1, false>(dim3(1, Hkv, num_seqs), q, k_pages, v_pages, out, nullptr, q_start, kv_len,
+                                        block_table, table_stride, page_size, num_pages, Hq, Hkv, scale, window, 0, status,
+                                        stream);
+#define Q3_AF_WHOLE(RPT)                                                                                                   \
+  return attn_f32_launch<D, RPT, false>(dim3((max_q_len + 8 * RPT / G - 1) / (8 * RPT / G), Hkv, num_seqs), q, k_pages,     \
+                                        v_pages, out, nullptr, q_start, kv_len, block_table, table_stride, page_size,       \
+                                        num_pages, Hq, Hkv, scale, window, 0, status, stream)
+  // 16 rows per block where blocks of 32 would leave SMs without one (37 tokens over 1,000 keys: 143 against 184 us), else
+  // 32 (prompts of 203 and 310 tokens: 76 us against 90 with 16 rows, and 111 with 64, whose one warp per scheduler waits
+  // for every shared-memory read)
+  if ((long long)((max_q_len + 32 / G - 1) / (32 / G)) * Hkv * num_seqs < sm_count()) Q3_AF_WHOLE(2);
+  Q3_AF_WHOLE(4);
+#undef Q3_AF_WHOLE
+}
+
+}  // namespace q3
+
+// float32; q, out: [T, Hq, D] with D 64 or 128; k_pages / v_pages: [num_pages, Hkv, page_size, D]; Hq / Hkv 1, 2, 4 or 8.
+// q_start: int32 [num_seqs + 1]; kv_len: int32 [num_seqs] keys after this step's write; block_table: int32 [num_seqs,
+// table_stride].  max_chunks > 0: every request brings one token, none has more than 64 max_chunks keys, and partial holds
+// num_seqs * Hq * max_chunks * (D + 4) floats; 0: requests of up to max_q_len tokens, partial not used.  The results are
+// the same bits either way.  window <= 0: all earlier keys.
+extern "C" int q3_attn_f32(const float* q, const float* k_pages, const float* v_pages, float* out, float* partial,
+                           const int* q_start, const int* kv_len, const int* block_table, int table_stride, int page_size,
+                           int num_pages, int num_seqs, int max_q_len, int Hq, int Hkv, int D, float scale, int window,
+                           int max_chunks, int* status, cudaStream_t stream) {
+  if (num_seqs <= 0 || max_q_len <= 0) return 0;
+  if (Hkv <= 0 || Hq % Hkv || page_size <= 0 || table_stride <= 0 || max_chunks < 0 || (max_chunks > 0 && !partial))
+    return Q3_ERR_SIZE;
+  const int G = Hq / Hkv;
+  if ((G != 1 && G != 2 && G != 4 && G != 8) || Hkv > 65535 || num_seqs > 65535) return Q3_ERR_SIZE;
+  if ((uintptr_t)q % 16 || (uintptr_t)k_pages % 16 || (uintptr_t)v_pages % 16 || (uintptr_t)out % 16 || (uintptr_t)partial % 16)
+    return Q3_ERR_ALIGN;
+#define Q3_AF_GO(D_)                                                                                                        \
+  return q3::attn_f32_go<D_>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride, page_size,      \
+                             num_pages, num_seqs, max_q_len, Hq, Hkv, scale, window, max_chunks, status, stream)
+  if (D == 64) Q3_AF_GO(64);
+  if (D == 128) Q3_AF_GO(128);
+#undef Q3_AF_GO
+  return Q3_ERR_SIZE;
+}

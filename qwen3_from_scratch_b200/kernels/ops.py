@@ -55,6 +55,8 @@ _SIGNATURES = {
     "q3_attn_ref": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                     _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
                     _c_void_p, _c_void_p],
+    "q3_attn_f32": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
+                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void_p, _c_void_p],
     "q3_attn_decode": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                        _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int,
                        _c_void_p, _c_void_p],
@@ -893,6 +895,51 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages: 
     _done("gemm_tc_qkv", code, f"T {T} K {K} heads {num_q_heads}/{num_kv_heads} x {head_dim}{' pair' if pair else ''}")
 
 
+def attn_f32_takes(dtype: torch.dtype, num_q_heads: int, num_kv_heads: int, head_dim: int) -> bool:
+    """Whether the float32 chunk kernels take this shape (else the plain kernel runs)."""
+    return (dtype == torch.float32 and head_dim in (64, 128) and num_q_heads % num_kv_heads == 0
+            and num_q_heads // num_kv_heads in (1, 2, 4, 8))
+
+
+ATTN_F32_CHUNK = 64        # keys per chunk: part of the order of a query's additions, not a tuning knob
+ATTN_F32_SCRATCH_CHUNKS = 64
+ATTN_F32_SCRATCH = 1 << 24  # floats
+
+
+def attn_f32_partial_numel(num_seqs: int, num_q_heads: int, head_dim: int) -> int:
+    """Scratch for single tokens: contexts of 4,096 tokens for all ``num_seqs`` requests at once, up to 64 MB."""
+    return min(num_seqs * num_q_heads * ATTN_F32_SCRATCH_CHUNKS * (head_dim + 4), ATTN_F32_SCRATCH)
+
+
+def attn_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
+             kv_len: torch.Tensor, block_table: torch.Tensor, num_seqs: int, max_q_len: int, max_kv_len: int, scale: float,
+             window: int, status: torch.Tensor, partial: Optional[torch.Tensor] = None) -> None:
+    """float32 attention by chunks of 64 keys (csrc/attn_f32.cu).  Requests of a single token run their chunks side by
+    side where ``partial`` holds all of them (longer contexts than the scratch was made for are walked by one block per
+    request and kv head); the results are the same bits either way."""
+    T, Hq, D = q.shape
+    num_pages, Hkv, page_size, d = k_pages.shape
+    for name, t in (("q", q), ("k_pages", k_pages), ("v_pages", v_pages), ("out", out)):
+        _check(f"attn_f32.{name}", t, torch.float32)
+    for name, t in (("q_start", q_start), ("kv_len", kv_len), ("block_table", block_table)):
+        _check(f"attn_f32.{name}", t, torch.int32)
+    if d != D or v_pages.shape != k_pages.shape or out.numel() != q.numel() or block_table.dim() != 2:
+        raise KernelError(f"attn_f32: q {tuple(q.shape)}, pages {tuple(k_pages.shape)}, out {tuple(out.shape)}")
+    if num_seqs > kv_len.numel() or num_seqs > block_table.shape[0] or num_seqs >= q_start.numel():
+        raise KernelError(f"attn_f32: {num_seqs} sequences, {kv_len.numel()} lengths")
+    chunks = 0
+    if max_q_len == 1 and partial is not None:
+        _check("attn_f32.partial", partial, torch.float32)
+        chunks = -(-max_kv_len // ATTN_F32_CHUNK)
+        if partial.numel() < num_seqs * Hq * chunks * (D + 4):
+            chunks = 0
+    code = library().q3_attn_f32(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(),
+                                 _ptr(partial) if chunks else None, q_start.data_ptr(), kv_len.data_ptr(),
+                                 block_table.data_ptr(), block_table.shape[1], page_size, num_pages, num_seqs, max_q_len, Hq,
+                                 Hkv, D, float(scale), int(window), chunks, status.data_ptr(), _stream())
+    _done("attn_f32", code, f"heads {Hq}/{Hkv}, head_dim {D}")
+
+
 def fast_attention_takes(dtype: torch.dtype, num_q_heads: int, num_kv_heads: int, head_dim: int) -> bool:
     """Whether the tensor-core kernels take this shape (else the plain kernel runs)."""
     return (dtype == torch.bfloat16 and head_dim % 16 == 0 and 16 <= head_dim <= 256
@@ -1159,13 +1206,21 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     """``raw_qkv``: see ``attn_decode``; only where ``decode_takes_raw_qkv`` says so.
     Causal attention of a mixed batch over the pages: rows [0, num_decode) bring one token each and
     go to the split-KV decode kernel, the rest to a portion kernel (tcgen05 where it takes the shape,
-    else mma.sync; ``portion_kernel="mma"`` forces the latter); shapes no tensor-core kernel takes
-    (and float32) go to the plain kernel."""
+    else mma.sync; ``portion_kernel="mma"`` forces the latter).  float32 goes to the chunk kernels of csrc/attn_f32.cu
+    (head sizes 64 and 128, up to 8 query heads per kv head); shapes that none of these takes go to the plain kernel."""
     T, Hq, D = q.shape
     Hkv = k_pages.shape[1]
     if block_table.dim() != 2 or max_kv_len > block_table.shape[1] * k_pages.shape[2]:
         raise KernelError(f"paged_attention: the longest request has {max_kv_len} tokens, a block table row of "
                           f"{block_table.shape[-1]} pages of {k_pages.shape[2]} holds fewer")
+    if attn_f32_takes(q.dtype, Hq, Hkv, D):
+        if num_decode > 0:
+            attn_f32(q, k_pages, v_pages, out, q_start, kv_len, block_table, num_decode, 1, max_kv_len, scale, window,
+                     status, partial)
+        if num_seqs > num_decode:
+            attn_f32(q, k_pages, v_pages, out, q_start[num_decode:], kv_len[num_decode:], block_table[num_decode:],
+                     num_seqs - num_decode, max_q_len, max_kv_len, scale, window, status)
+        return
     if not fast_attention_takes(q.dtype, Hq, Hkv, D):
         attn_ref(q, k_pages, v_pages, out, q_start, kv_len, tok_seq, block_table, scale, window, status)
         return

@@ -185,6 +185,66 @@ def test_gemm_f32_orders_agree(N, K):
         assert torch.equal(wide[:, :N], out[:M]) and bool(torch.isnan(wide[:, N:]).all()), M
 
 
+@pytest.mark.parametrize("hq,hkv,d,page_size,window", [(16, 8, 128, 16, None), (8, 1, 64, 8, None), (4, 4, 128, 16, 70),
+                                                       (8, 2, 64, 32, 1)])
+def test_attn_f32(hq, hkv, d, page_size, window):
+    """Float32 attention by chunks of 64 keys: lengths around a chunk's and a page's edges, portions that begin inside a
+    chunk, single tokens side by side and walked, all against float64; every cut gives the same bits."""
+    o = ops()
+    lens = [1, 63, 64, 65, 129, 200, 300, 8]
+    q, k_list, v_list, tables, num_pages = attention_case("float32", hq, hkv, d, page_size, lens, lens, window, seed=31)
+    kp, vp = (dev(paged(x, page_size, tables, num_pages, torch.float32)) for x in (k_list, v_list))
+    want = reference_attention(q.double(), [k.double() for k in k_list], [v.double() for v in v_list], lens, window)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    Q, table = dev(q), dev(table_tensor(tables))
+
+    def run(cuts, max_kv, partial=None):
+        """cuts: (tokens before, tokens of the step) per request; rows of the whole result."""
+        qs = torch.cat([Q[starts[i] + b:starts[i] + b + n] for i, (b, n) in enumerate(cuts)])
+        out, st = torch.full_like(qs, float("nan")), status()
+        q_start = dev(torch.tensor([sum(n for _, n in cuts[:i]) for i in range(len(cuts) + 1)], dtype=torch.int32))
+        o.attn_f32(qs, kp, vp, out, q_start, dev(torch.tensor([b + n for b, n in cuts], dtype=torch.int32)), table, len(cuts),
+                   max(n for _, n in cuts), max_kv, d ** -0.5, window or 0, st, partial)
+        assert int(st.item()) == 0
+        return out
+
+    whole = run([(0, n) for n in lens], max(lens))
+    close(whole, want, "float32")
+    # a portion's first and last token, and tokens in between
+    for cuts in ([(n // 2, n - n // 2) for n in lens], [(n - min(n, 5), min(n, 5)) for n in lens]):
+        out = run(cuts, max(lens))
+        assert torch.equal(out, torch.cat([whole[starts[i] + b:starts[i] + b + n] for i, (b, n) in enumerate(cuts)]))
+    last = torch.stack([whole[s + n - 1] for s, n in zip(starts, lens)])
+    single = [(n - 1, 1) for n in lens]
+    partial = torch.full((o.attn_f32_partial_numel(len(lens), hq, d),), float("nan"), device="cuda")
+    assert torch.equal(run(single, max(lens), partial), last)
+    assert torch.equal(run(single, 1024, partial), last)  # more chunks than any request has
+    assert torch.equal(run(single, max(lens)), last)      # no scratch: walked
+
+
+def test_attn_f32_reports_bad_tables():
+    """A page outside the pool and a context beyond what the launch was made for are reported, not read; a value that a
+    query does not see takes no part in its sum, even if it is not a number."""
+    o = ops()
+    hq, hkv, d, page_size, n = 4, 2, 64, 16, 100
+    q, k_list, v_list, tables, num_pages = attention_case("float32", hq, hkv, d, page_size, [n], [n], None, seed=32)
+    v_list[0][70] = float("nan")
+    kp, vp = (dev(paged(x, page_size, tables, num_pages, torch.float32)) for x in (k_list, v_list))
+    table, lens = dev(table_tensor(tables)), dev(torch.tensor([n], dtype=torch.int32))
+    out, st = torch.empty_like(dev(q)), status()
+    o.attn_f32(dev(q), kp, vp, out, dev(torch.tensor([0, n], dtype=torch.int32)), lens, table, 1, n, n, d ** -0.5, 0, st)
+    assert int(st.item()) == 0 and not bool(torch.isnan(out[:70]).any()) and bool(torch.isnan(out[70:]).all())
+    one, partial = dev(q)[-1:].contiguous(), torch.empty(o.attn_f32_partial_numel(1, hq, d), device="cuda")
+    single = dev(torch.tensor([0, 1], dtype=torch.int32))
+    bad = table.clone()
+    bad[0, 4] = num_pages + 7  # keys 64 .. 79: left out, the 100th value of key 70 with them
+    o.attn_f32(one, kp, vp, out[:1], single, lens, bad, 1, 1, n, d ** -0.5, 0, st, partial)
+    assert int(st.item()) == 2 and not bool(torch.isnan(out[0]).any())
+    st.zero_()
+    o.attn_f32(one, kp, vp, out[:1], single, lens, table, 1, 1, 64, d ** -0.5, 0, st, partial)
+    assert int(st.item()) == 4
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 def test_swiglu(dtype):
     g = torch.Generator().manual_seed(4)
