@@ -55,6 +55,11 @@ _SIGNATURES = {
     "q3_attn_ref": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                     _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
                     _c_void_p, _c_void_p],
+    "q3_latent_gather": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+                         _c_void_p, _c_void_p, _c_void_p, _c_void_p],
+    "q3_latent_attn_tc": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
+                          _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
+    "q3_latent_attn_tc_wait_test": [ctypes.c_uint, _c_int],
     "q3_attn_f32": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
                     _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void_p, _c_void_p],
     "q3_attn_decode": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
@@ -1940,6 +1945,69 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Te
         _ptr(partial) if splits > 1 else None, T, ctx.num_seqs, ctx.max_q_len, H, rank, rot, float(scale), splits,
         _ptr(sink), status.data_ptr(), _stream())
     _done("latent_attention (mma)", code, f"heads {H}, rank {rank}, rot {rot}, splits {splits}")
+
+
+def latent_formed_takes(dtype: torch.dtype, dim: int, rot: int, vdim: int, rank: int, scale: float) -> bool:
+    """Whether prompt portions can attend over formed keys and values (csrc/latent_attn_tc.cu)."""
+    return dtype == torch.bfloat16 and dim == 128 and vdim == 128 and rot == 64 and rank % 8 == 0 and scale > 0
+
+
+def latent_formed_rows(max_tokens: int) -> int:
+    """Rows of formed keys and values that scratch is laid out for."""
+    return max(int(max_tokens), LATENT_FORMED_ROWS)
+
+
+def latent_formed_pays(ctx, capacity: int) -> bool:
+    """Whether a step's requests attend over formed keys and values: portions only, whose rows (the longest context's, per
+    request) fit the scratch, with enough tokens per row for the forming.  Forming costs about 6 ns a row, the absorbed
+    kernel 0.25 ns per token and key more than the formed one, so from some 24 tokens per request on; measured on whole
+    steps of 12 layers (absorbed / formed us): 40 tokens 1,367 / 1,279, 40 + 50 + 60 tokens 1,829 / 1,786, 400 tokens
+    1,856 / 1,516, 2,048 tokens 7,410 / 4,305."""
+    rows = ctx.num_seqs * ctx.max_kv_len
+    return ctx.num_decode == 0 and rows <= capacity and ctx.positions.numel() * LATENT_FORMED_ROWS_PER_TOKEN >= rows
+
+
+LATENT_FORMED_ROWS = 4096
+LATENT_FORMED_ROWS_PER_TOKEN = 32  # a context's length is rounded up to 1,024 for the rows
+
+
+def latent_attention_formed(q_plain: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Tensor, r_pages: torch.Tensor, ctx,
+                            table: torch.Tensor, kv_up_t: torch.Tensor, c_rows: torch.Tensor, r_rows: torch.Tensor,
+                            kv: torch.Tensor, out: torch.Tensor, scale: float, status: torch.Tensor,
+                            gate: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None) -> None:
+    """Latent attention of prompt portions with every head's keys and values formed first: the latents of all keys are
+    brought out of their pages into ``c_rows`` / ``r_rows``, one product with ``kv_up_t`` [rank, 2 H 128] (the transposed
+    W_uk and W_uv of all heads) makes ``kv``, and out [T, H * 128] = gate * softmax attention of q_plain [T, H * 128] and
+    q_rot [T, H, 64] over it."""
+    T, H, rot = q_rot.shape
+    rank = c_pages.shape[3]
+    for name, t in (("q_plain", q_plain), ("q_rot", q_rot), ("c_pages", c_pages), ("r_pages", r_pages), ("c_rows", c_rows),
+                    ("r_rows", r_rows), ("kv", kv), ("out", out)):
+        _check(f"latent_attention_formed.{name}", t, torch.bfloat16)
+    for name, t in (("q_start", ctx.q_start), ("kv_len", ctx.kv_len), ("table", table)):
+        _check(f"latent_attention_formed.{name}", t, torch.int32)
+    for name, t, n in (("gate", gate, T * H), ("sink", sink, H)):
+        if t is not None:
+            _check(f"latent_attention_formed.{name}", t, torch.float32)
+            if t.numel() != n:
+                raise KernelError(f"latent_attention_formed: {name} has {t.numel()} values, {n} expected")
+    pitch, B = ctx.max_kv_len, ctx.num_seqs
+    rows = B * pitch
+    if (q_plain.numel() != T * H * 128 or rot != 64 or out.numel() != T * H * 128 or tuple(kv_up_t.shape) != (rank, 2 * H * 128)
+            or c_rows.shape[0] < rows or c_rows.shape[1] != rank or r_rows.shape[0] < rows or r_rows.shape[1] != rot
+            or kv.shape[0] < rows or kv.shape[1] != 2 * H * 128 or c_pages.shape[1] != 1 or r_pages.shape[3] != rot
+            or r_pages.shape[:3] != c_pages.shape[:3] or ctx.kv_len.numel() < B or table.shape[0] < B):
+        raise KernelError(f"latent_attention_formed: q_plain {tuple(q_plain.shape)}, q_rot {tuple(q_rot.shape)}, c "
+                          f"{tuple(c_pages.shape)}, r {tuple(r_pages.shape)}, kv {tuple(kv.shape)}, {B} requests of {pitch} rows")
+    code = library().q3_latent_gather(c_pages.data_ptr(), r_pages.data_ptr(), ctx.kv_len.data_ptr(), table.data_ptr(),
+                                      table.shape[1], c_pages.shape[2], c_pages.shape[0], B, pitch, rank, rot,
+                                      c_rows.data_ptr(), r_rows.data_ptr(), status.data_ptr(), _stream())
+    _done("latent_gather", code, f"rank {rank}, rot {rot}, {B} requests of {pitch} rows")
+    torch.mm(c_rows[:rows], kv_up_t, out=kv[:rows])
+    code = library().q3_latent_attn_tc(q_plain.data_ptr(), q_rot.data_ptr(), kv.data_ptr(), r_rows.data_ptr(), out.data_ptr(),
+                                       ctx.q_start.data_ptr(), ctx.kv_len.data_ptr(), B, pitch, ctx.max_q_len, H, float(scale),
+                                       _ptr(gate), _ptr(sink), status.data_ptr(), _stream())
+    _done("latent_attn_tc", code, f"{H} heads, {B} requests of {pitch} rows")
 
 
 # ------------------------------------------------------------------ layer norm and the convolution before a sub-layer

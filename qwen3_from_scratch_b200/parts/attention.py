@@ -314,6 +314,14 @@ class LatentAttention(Mixer):
         # the attended latent out; both in the compute dtype (a float32 run: float32)
         self.uk_t = uk.view(H, self.dim, self.kv_rank).transpose(1, 2).to(rt.dtype).contiguous()
         self.uv = uv.view(H, self.vdim, self.kv_rank).to(rt.dtype).contiguous()
+        # prompt portions form the heads' keys and values instead: both weights as one product over the latents
+        self.formed = ops.latent_formed_takes(rt.dtype, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.scale)
+        if self.formed:
+            self.kv_up_t = torch.cat([uk.to(rt.dtype), uv.to(rt.dtype)], dim=0).t()
+            rows = ops.latent_formed_rows(rt.max_tokens)
+            self._c_rows = rt.shared("lattn.c_rows", rows, self.kv_rank)
+            self._r_rows = rt.shared("lattn.r_rows", rows, self.rot_dim)
+            self._kv = rt.shared("lattn.kv", rows, 2 * H * self.dim)
         del uk, uv
         self.o_proj = Linear(weights.pop(t["out"]), rt, tag="lattn.o_proj")
         self.position.setup(rt, weights)
@@ -344,6 +352,11 @@ class LatentAttention(Mixer):
         q_plain, q_rot = self._q_plain[:T], self._q_rot[:T]
         ops.latent_q_post(self.up_q(cq), H, self.dim, rot, dims, freq, mag, ctx.positions, q_plain, q_rot,
                           pairing=self.pairing)
+        out = self._o[:T]
+        if self.formed and ops.latent_formed_pays(ctx, self._kv.shape[0]):
+            ops.latent_attention_formed(q_plain, q_rot, c_pages, r_pages, ctx, table, self.kv_up_t, self._c_rows, self._r_rows,
+                                        self._kv, out, self.scale, status, gate=gate, sink=self.sink)
+            return self.o_proj(out)
         q_abs = self._q_abs[: H * T * rank].view(H, T, rank)
         ops.block_diag(q_plain, self.uk_t, q_abs)
         o_lat = self._o_lat[:T]
@@ -351,7 +364,6 @@ class LatentAttention(Mixer):
                              sink=self.sink)
         o_heads = self._o_heads[: H * T * self.vdim].view(H, T, self.vdim)
         ops.block_diag(o_lat, self.uv, o_heads)
-        out = self._o[:T]
         ops.gate_heads(o_heads, gate, out)
         return self.o_proj(out)
 

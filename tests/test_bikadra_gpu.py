@@ -450,6 +450,67 @@ def replay(folder, dtype, seqs, schedule, **session_args):
     return r.result()
 
 
+@pytest.mark.parametrize("H,rank,page,gated,sink,pitch", [(3, 64, 16, True, False, 512), (2, 512, 8, False, True, 300),
+                                                          (17, 128, 16, True, True, 1024)])
+def test_latent_attention_over_formed_keys(H, rank, page, gated, sink, pitch):
+    """Portions over formed keys and values against float64 on the same latents: requests that begin in the cache and
+    whole ones, lengths around the 128 rows and keys of a tile, pages in another order than the tokens'.  What lies
+    behind a request's keys (rows never written, another request's rows) holds NaN."""
+    from types import SimpleNamespace
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(H * 1000 + rank)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    bf = lambda t: t.to(torch.bfloat16).cuda()  # noqa: E731
+    q_lens, kv_lens = [128, 70, 1, 129, 3, 40, 1], [128, 200, 77, 129, 259, 296, 1]
+    B, T, rot, d = len(q_lens), sum(q_lens), 64, 128
+    need = [-(-n // page) for n in kv_lens]
+    order = torch.randperm(sum(need) + 3, generator=g).tolist()
+    table, at = torch.full((B, max(need) + 1), -1, dtype=torch.int32), 0
+    for b, n in enumerate(need):
+        table[b, :n] = torch.tensor(order[at:at + n], dtype=torch.int32)
+        at += n
+    c_pages, r_pages = (torch.full((len(order), 1, page, n), float("nan"), dtype=torch.bfloat16, device="cuda") for n in (rank, rot))
+    lat, rots = [], []
+    for b, n in enumerate(kv_lens):
+        lat.append(bf(torch.randn(n, rank, generator=g)))
+        rots.append(bf(torch.randn(n, rot, generator=g)))
+        for i in range(n):
+            c_pages[table[b, i // page], 0, i % page] = lat[b][i]
+            r_pages[table[b, i // page], 0, i % page] = rots[b][i]
+    q_plain, q_rot = bf(torch.randn(T, H * d, generator=g) * 0.5), bf(torch.randn(T, H, rot, generator=g) * 0.5)
+    up = bf(torch.randn(2 * H * d, rank, generator=g) * rank ** -0.5)
+    gate = torch.rand(T, H, generator=g).cuda() if gated else None
+    sinks = torch.randn(H, generator=g).cuda() if sink else None
+    ctx = SimpleNamespace(positions=i32([0] * T), q_start=i32([0] + torch.tensor(q_lens).cumsum(0).tolist()), kv_len=i32(kv_lens),
+                          num_seqs=B, num_decode=0, max_q_len=max(q_lens), max_kv_len=pitch)
+    c_rows, r_rows, kv = (torch.full((B * pitch + 5, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+                          for n in (rank, rot, 2 * H * d))
+    out, status, scale = torch.full((T, H * d), float("nan"), dtype=torch.bfloat16, device="cuda"), i32([0]), (d + rot) ** -0.5
+    ops.latent_attention_formed(q_plain, q_rot, c_pages, r_pages, ctx, table.cuda(), up.t(), c_rows, r_rows, kv, out, scale,
+                                status, gate=gate, sink=sinks)
+    assert int(status.item()) == 0
+    at, wants = 0, []
+    for b, (n, total) in enumerate(zip(q_lens, kv_lens)):
+        formed = lat[b].double() @ up.double().t()
+        k, v = formed[:, :H * d].view(total, H, d), formed[:, H * d:].view(total, H, d)
+        s = torch.einsum("thd,nhd->htn", q_plain[at:at + n].double().view(n, H, d), k)
+        s = (s + torch.einsum("thd,nd->htn", q_rot[at:at + n].double(), rots[b].double())) * scale
+        hidden = torch.arange(total, device="cuda")[None] > torch.arange(total - n, total, device="cuda")[:, None]
+        s = s.masked_fill(hidden, -float("inf"))
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(H, n, 1)], dim=-1)
+        w = s.softmax(-1)[..., :total]
+        o = torch.einsum("htn,nhd->thd", w, v)
+        wants.append(o * gate[at:at + n].double()[..., None] if gated else o)
+        at += n
+    want = torch.cat(wants).view(T, H * d)
+    # keys, values, weights and the result are each rounded to bfloat16 once (2^-9 of the largest value apiece)
+    assert float((out.double() - want).abs().max()) <= 4 * 2.0 ** -9 * float(want.abs().max())
+    ctx.kv_len, ctx.max_kv_len = i32([n + 4096 for n in kv_lens]), 64  # more keys than rows: reported, nothing read
+    ops.latent_attention_formed(q_plain, q_rot, c_pages, r_pages, ctx, table.cuda(), up.t(), c_rows, r_rows, kv, out, scale, status)
+    assert int(status.item()) & 4
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 @pytest.mark.parametrize("key", list(CONFIGS))
 def test_model_whole_decoded_and_in_portions(folders, key, dtype):
