@@ -9,11 +9,11 @@
 // and the chunks are folded together in ascending order: m' = max(m, m_c), l' = l exp(m - m') + l_c exp(m_c - m'), o likewise.
 // Long contexts keep their accuracy (sums of 64, then one term per chunk), and the chunks of a single token can be
 // computed side by side:
-//   attn_f32_kernel, whole      a block takes 16 or 32 (token, head) rows of one kv head and walks over the chunks
-//   attn_f32_kernel, by chunks  a block takes the heads of one token and one chunk and leaves (m_c, l_c, o_c)
-//   attn_f32_fold_kernel        folds them
-// Sizes of the 0.6B model (16 heads over 8 of 128), cold caches: 4 single tokens at contexts of 400 to 900 31.7 us, one at
-// 4,096 69 us, prompts of 203 and 310 tokens 76 us; the walk over the keys one by one that served here before (attn_ref.cu,
+//   attn_f32_kernel        a block takes up to 32 (token, head) rows of one kv head and walks over the chunks
+//   attn_f32_chunk_kernel  a block takes the heads of one token and one chunk and leaves (m_c, l_c, o_c)
+//   attn_f32_fold_kernel   folds them
+// Sizes of the 0.6B model (16 heads over 8 of 128), cold caches: 4 single tokens at contexts of 400 to 900 23.6 us, one at
+// 4,096 36 us, prompts of 203 and 310 tokens 76 us; the walk over the keys one by one that served here before (attn_ref.cu,
 // a warp per token and head) took 1,435, 6,600 and 453 us: some 1.6 us per key of the longest context, whatever the batch.
 //
 // Reference formulas: as in attn_ref.cu (models/attn.py:402-499, kernels/triton/paged_attn.py:89-181).
@@ -37,15 +37,15 @@ struct AfShape {
   static constexpr size_t SMEM = ((size_t)(ROWS + 2 * AF_CHUNK) * D + (size_t)ROWS * AF_CHUNK) * sizeof(float);
 };
 
-// BY_CHUNK: grid (chunks, kv heads, requests), single-token requests only; else grid (token tiles, kv heads, requests).
+// Grid (token tiles, kv heads, requests).
 // Bound by shared-memory reads and the FMA pipe together (a 4 x 4 piece of the scores per thread: 8 reads of 16 bytes for
 // 64 FMA); K of the next chunk is fetched under P V, V under the scores.
-template <int D, int RPT, bool BY_CHUNK>
+template <int D, int RPT>
 __global__ void __launch_bounds__(AF_THREADS)
 attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
-                float* __restrict__ out, float* __restrict__ partial, const int* __restrict__ q_start,
-                const int* __restrict__ kv_len, const int* __restrict__ block_table, int table_stride, int page_size,
-                int num_pages, int Hq, int Hkv, float scale, int window, int max_chunks, int* status) {
+                float* __restrict__ out, const int* __restrict__ q_start, const int* __restrict__ kv_len,
+                const int* __restrict__ block_table, int table_stride, int page_size, int num_pages, int Hq, int Hkv,
+                float scale, int window, int* status) {
   constexpr int ROWS = 8 * RPT, D4 = D / 4, DV = D / 64;  // DV: pieces of four output columns per thread
   pdl_wait();
   pdl_launch_dependents();
@@ -59,15 +59,14 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;  // rows ty + 8 i, keys tx + 16 j
   const int b = blockIdx.z, hk = blockIdx.y, G = Hq / Hkv;
   const int t0 = q_start[b], q_len = q_start[b + 1] - t0, len = kv_len[b];
-  const int tokens = ROWS / G, tok0 = BY_CHUNK ? 0 : blockIdx.x * tokens;
+  const int tokens = ROWS / G, tok0 = blockIdx.x * tokens;
   if (tok0 >= q_len) return;
   const int live_rows = min(tokens, q_len - tok0) * G;
   const int first_pos = len - q_len + tok0, last_pos = first_pos + min(tokens, q_len - tok0) - 1;
   const int first_key = (window > 0 && first_pos - window + 1 > 0) ? first_pos - window + 1 : 0;
-  int chunk = BY_CHUNK ? blockIdx.x : first_key / AF_CHUNK;
-  const int chunk_end = BY_CHUNK ? chunk + 1 : last_pos / AF_CHUNK + 1;
-  if (first_pos < 0 && tid == 0 && (!BY_CHUNK || chunk == 0)) atomicOr(status, Q3_STATUS_BAD_POSITION);
-  if (BY_CHUNK && (chunk * AF_CHUNK > last_pos || (chunk + 1) * AF_CHUNK <= first_key)) return;
+  int chunk = first_key / AF_CHUNK;
+  const int chunk_end = last_pos / AF_CHUNK + 1;
+  if (first_pos < 0 && tid == 0) atomicOr(status, Q3_STATUS_BAD_POSITION);
 
   for (int e = tid; e < ROWS * D4; e += AF_THREADS) {
     const int r = e / D4, c = e % D4;
@@ -166,7 +165,7 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
         for (int j = 0; j < 4; ++j) {
           const int key = tx + 16 * j, n = chunk * AF_CHUNK + key;
           sees[j] = n >= lo[i] && n <= pos[i] && ((ok >> key) & 1ull);
-          s[i][j] *= scale;
+          s[i][j] = __fmul_rn(s[i][j], scale);  // (not contracted with the subtraction below)
           if (sees[j]) mc[i] = fmaxf(mc[i], s[i][j]);
         }
 #pragma unroll
@@ -220,16 +219,7 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
     }
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
-      const int r = ty + 8 * i;
-      if constexpr (BY_CHUNK) {
-        if (r >= live_rows) continue;
-        float* dst = partial + ((size_t)(b * Hq + hk * G + r) * max_chunks + chunk) * (D + 4);
-#pragma unroll
-        for (int c = 0; c < DV; ++c)
-          *reinterpret_cast<float4*>(dst + (tx + 16 * c) * 4) =
-              make_float4(oc[i][4 * c], oc[i][4 * c + 1], oc[i][4 * c + 2], oc[i][4 * c + 3]);
-        if (tx == 0) *reinterpret_cast<float4*>(dst + D) = make_float4(mc[i], lc[i], 0.f, 0.f);
-      } else if (!(mc[i] == -INFINITY && lc[i] == 0.f)) {  // else: no key of the chunk is seen
+      if (!(mc[i] == -INFINITY && lc[i] == 0.f)) {  // else: no key of the chunk is seen
         const float mn = fmaxf(m[i], mc[i]), f = expf(m[i] - mn), g = expf(mc[i] - mn);
         l[i] = fmaf(l[i], f, lc[i] * g);
 #pragma unroll
@@ -238,18 +228,154 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
       }
     }
   }
-  if constexpr (!BY_CHUNK) {
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      const int r = ty + 8 * i;
-      if (r >= live_rows) continue;
-      const float inv = l[i] == 0.f ? 0.f : 1.0f / l[i];
-      float* dst = out + ((size_t)(t0 + tok0 + r / G) * Hq + hk * G + r % G) * D;
+  for (int i = 0; i < RPT; ++i) {
+    const int r = ty + 8 * i;
+    if (r >= live_rows) continue;
+    const float inv = l[i] == 0.f ? 0.f : 1.0f / l[i];
+    float* dst = out + ((size_t)(t0 + tok0 + r / G) * Hq + hk * G + r % G) * D;
 #pragma unroll
-      for (int c = 0; c < DV; ++c)
-        *reinterpret_cast<float4*>(dst + (tx + 16 * c) * 4) =
-            make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+    for (int c = 0; c < DV; ++c)
+      *reinterpret_cast<float4*>(dst + (tx + 16 * c) * 4) =
+          make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+  }
+}
+
+// Single tokens: grid (chunks, kv heads, requests), the G heads of one kv head against one chunk; leaves o_c, m_c and l_c of
+// each head.  The same additions in the same order as above, shared out so that all four warps work whatever G is: a
+// thread per key (and every second head) for the scores, a half-warp per head for the softmax, a thread per output
+// column for P V (4 requests at contexts of 400 to 900, 16 heads over 8 of 128: 14.5 us with the kernel above cut by chunks,
+// one of whose warps had rows, 13.0 us here; batch 1 at 4,096: 69 and 36 us with the fold).
+template <int D, int G>
+__global__ void __launch_bounds__(AF_THREADS)
+attn_f32_chunk_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                      float* __restrict__ partial, const int* __restrict__ q_start, const int* __restrict__ kv_len,
+                      const int* __restrict__ block_table, int table_stride, int page_size, int num_pages, int Hq, int Hkv,
+                      float scale, int window, int max_chunks, int* status) {
+  constexpr int D4 = D / 4;
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(128) float af_smem[];
+  float* k_s = af_smem;                  // [64][D], piece c of a row at place c ^ (row & 7)
+  float* v_s = k_s + AF_CHUNK * D;       // [64][D], as it is
+  __shared__ __align__(16) float q_s[G][D];
+  __shared__ __align__(16) float p_s[8][AF_CHUNK];
+  __shared__ unsigned long long key_ok;  // bit n: key n of the chunk has a page
+  const int tid = threadIdx.x, b = blockIdx.z, hk = blockIdx.y, chunk = blockIdx.x;
+  const int t = q_start[b], pos = kv_len[b] - 1;
+  if (q_start[b + 1] == t) return;
+  if (pos < 0 && tid == 0 && chunk == 0) atomicOr(status, Q3_STATUS_BAD_POSITION);
+  const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  if (chunk * AF_CHUNK > pos || (chunk + 1) * AF_CHUNK <= lo) return;
+  if (tid == 0) key_ok = 0ull;
+
+  const int my_key = tid >> 1, n_mine = chunk * AF_CHUNK + my_key;  // two threads per key bring its rows
+  int page = -1;
+  if (n_mine >= lo && n_mine <= pos) {
+    page = table_page(block_table + (size_t)b * table_stride, n_mine / page_size, table_stride, status);
+    if (page < 0 || page >= num_pages) {
+      atomicOr(status, Q3_STATUS_BAD_PAGE);
+      page = -1;
     }
+  }
+  const size_t row = page < 0 ? 0 : (((size_t)page * Hkv + hk) * page_size + n_mine % page_size) * D;
+  const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(k_s), v_addr = (uint32_t)__cvta_generic_to_shared(v_s);
+#pragma unroll
+  for (int i = 0; i < D4 / 2; ++i) {
+    const int piece = 2 * i + (tid & 1);
+    af_copy16(k_addr + (my_key * D + (piece ^ (my_key & 7)) * 4) * 4, k_pages + row + piece * 4, page >= 0);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < D4 / 2; ++i) {
+    const int piece = 2 * i + (tid & 1);
+    af_copy16(v_addr + (my_key * D + piece * 4) * 4, v_pages + row + piece * 4, page >= 0);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int e = tid; e < G * D4; e += AF_THREADS)
+    *reinterpret_cast<float4*>(&q_s[e / D4][(e % D4) * 4]) =
+        af_lds(q + ((size_t)t * Hq + hk * G + e / D4) * D + (e % D4) * 4);
+  __syncthreads();
+  if (!(tid & 1) && page >= 0) atomicOr(&key_ok, 1ull << my_key);
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();  // K, Q, key_ok
+  const unsigned long long ok = key_ok;
+  {
+    constexpr int RH = (G + 1) / 2;  // heads of a thread: tid / 64, + 2, ..
+    const int key = tid & 63;
+    float s[RH];
+#pragma unroll
+    for (int i = 0; i < RH; ++i) s[i] = 0.f;
+#pragma unroll 2
+    for (int run = 0; run < D / 16; ++run) {
+      float part[RH];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 kv = af_lds(k_s + key * D + (((run * 4 + c) ^ (key & 7)) * 4));
+#pragma unroll
+        for (int i = 0; i < RH; ++i) {
+          const float4 a = af_lds(&q_s[min((tid >> 6) + 2 * i, G - 1)][(run * 4 + c) * 4]);
+          part[i] = c == 0 ? a.x * kv.x : fmaf(a.x, kv.x, part[i]);
+          part[i] = fmaf(a.y, kv.y, part[i]);
+          part[i] = fmaf(a.z, kv.z, part[i]);
+          part[i] = fmaf(a.w, kv.w, part[i]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RH; ++i) s[i] += part[i];
+    }
+#pragma unroll
+    for (int i = 0; i < RH; ++i)
+      if ((tid >> 6) + 2 * i < G) p_s[(tid >> 6) + 2 * i][key] = __fmul_rn(s[i], scale);
+  }
+  __syncthreads();
+  const int tx = tid & 15, head = tid >> 4;
+  float* dst = partial + ((size_t)(b * Hq + hk * G) * max_chunks + chunk) * (D + 4);
+  const size_t dst_pitch = (size_t)max_chunks * (D + 4);
+  if ((tid >> 5) * 2 < G) {  // whole warps, two heads each
+    float s[4], mc = -INFINITY, lc = 0.f;
+    bool sees[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int key = tx + 16 * j, n = chunk * AF_CHUNK + key;
+      s[j] = head < G ? p_s[head][key] : 0.f;
+      sees[j] = n >= lo && n <= pos && ((ok >> key) & 1ull);
+      if (sees[j]) mc = fmaxf(mc, s[j]);
+    }
+#pragma unroll
+    for (int x = 8; x > 0; x >>= 1) mc = fmaxf(mc, __shfl_xor_sync(0xffffffffu, mc, x));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float p = sees[j] ? expf(s[j] - mc) : AF_MASKED;
+      if (sees[j]) lc += p;
+      if (head < G) p_s[head][tx + 16 * j] = p;
+    }
+#pragma unroll
+    for (int x = 8; x > 0; x >>= 1) lc += __shfl_xor_sync(0xffffffffu, lc, x);
+    if (tx == 0 && head < G) *reinterpret_cast<float4*>(dst + head * dst_pitch + D) = make_float4(mc, lc, 0.f, 0.f);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();  // P and V
+  if (tid < D) {
+    float oc[G];
+#pragma unroll
+    for (int h = 0; h < G; ++h) oc[h] = 0.f;
+#pragma unroll 4
+    for (int n4 = 0; n4 < AF_CHUNK; n4 += 4) {
+      float v[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) v[n] = v_s[(n4 + n) * D + tid];
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        const float4 p4 = af_lds(&p_s[h][n4]);
+        const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+          if (!(p[n] < 0.f)) oc[h] = fmaf(p[n], v[n], oc[h]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < G; ++h) dst[h * dst_pitch + tid] = oc[h];
   }
 }
 
@@ -268,32 +394,58 @@ attn_f32_fold_kernel(const float* __restrict__ partial, float* __restrict__ out,
   float m = -INFINITY, l = 0.f, o = 0.f;
   const int end = min(pos / AF_CHUNK + 1, max_chunks);
   if (pos >= 0 && pos / AF_CHUNK >= max_chunks && d == 0) atomicOr(status, Q3_STATUS_BAD_POSITION);
+  constexpr int AT_ONCE = 8;  // chunks whose values are asked for together: the fold itself is a chain
   if (pos >= 0) {
-#pragma unroll 4
-    for (int c = lo / AF_CHUNK; c < end; ++c) {
-      const float* p = src + (size_t)c * (D + 4);
-      const float oc = p[d], mc = p[D], lc = p[D + 1];
-      if (mc == -INFINITY && lc == 0.f) continue;
-      const float mn = fmaxf(m, mc), f = expf(m - mn), g = expf(mc - mn);
-      l = fmaf(l, f, lc * g);
-      o = fmaf(o, f, oc * g);
-      m = mn;
+    for (int c0 = lo / AF_CHUNK; c0 < end; c0 += AT_ONCE) {
+      float oc[AT_ONCE];
+      float2 ml[AT_ONCE];
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) {
+        const float* p = src + (size_t)min(c0 + u, end - 1) * (D + 4);
+        oc[u] = p[d];
+        ml[u] = c0 + u < end ? *reinterpret_cast<const float2*>(p + D) : make_float2(-INFINITY, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) {
+        if (ml[u].x == -INFINITY && ml[u].y == 0.f) continue;
+        const float mn = fmaxf(m, ml[u].x), f = expf(m - mn), g = expf(ml[u].x - mn);
+        l = fmaf(l, f, ml[u].y * g);
+        o = fmaf(o, f, oc[u] * g);
+        m = mn;
+      }
     }
   }
   out[((size_t)t * Hq + head) * D + d] = l == 0.f ? 0.f : o * (1.0f / l);
 }
 
-template <int D, int RPT, bool BY_CHUNK>
-static int attn_f32_launch(dim3 grid, const float* q, const float* k_pages, const float* v_pages, float* out, float* partial,
+template <int D, int G>
+static int attn_f32_chunks(const float* q, const float* k_pages, const float* v_pages, float* out, float* partial,
                            const int* q_start, const int* kv_len, const int* block_table, int table_stride, int page_size,
-                           int num_pages, int Hq, int Hkv, float scale, int window, int max_chunks, int* status,
+                           int num_pages, int num_seqs, int Hq, int Hkv, float scale, int window, int max_chunks, int* status,
                            cudaStream_t stream) {
-  constexpr size_t smem = AfShape<D, RPT>::SMEM;
-  auto kernel = attn_f32_kernel<D, RPT, BY_CHUNK>;
+  constexpr size_t smem = (size_t)2 * AF_CHUNK * D * sizeof(float);
+  auto kernel = attn_f32_chunk_kernel<D, G>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  q3::launch(kernel, grid, dim3(AF_THREADS), smem, stream, q, k_pages, v_pages, out, partial, q_start, kv_len, block_table,
-             table_stride, page_size, num_pages, Hq, Hkv, scale, window, max_chunks, status);
+  q3::launch(kernel, dim3(max_chunks, Hkv, num_seqs), dim3(AF_THREADS), smem, stream, q, k_pages, v_pages, partial, q_start,
+             kv_len, block_table, table_stride, page_size, num_pages, Hq, Hkv, scale, window, max_chunks, status);
+  q3::launch(attn_f32_fold_kernel<D>, dim3(Hq, num_seqs), dim3(D), 0, stream, partial, out, q_start, kv_len, Hq, window,
+             max_chunks, status);
+  return launch_status();
+}
+
+template <int D, int RPT>
+static int attn_f32_walk(const float* q, const float* k_pages, const float* v_pages, float* out, const int* q_start,
+                         const int* kv_len, const int* block_table, int table_stride, int page_size, int num_pages,
+                         int num_seqs, int max_q_len, int Hq, int Hkv, float scale, int window, int* status,
+                         cudaStream_t stream) {
+  constexpr size_t smem = AfShape<D, RPT>::SMEM;
+  auto kernel = attn_f32_kernel<D, RPT>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  const int tokens = 8 * RPT / (Hq / Hkv);
+  q3::launch(kernel, dim3((max_q_len + tokens - 1) / tokens, Hkv, num_seqs), dim3(AF_THREADS), smem, stream, q, k_pages,
+             v_pages, out, q_start, kv_len, block_table, table_stride, page_size, num_pages, Hq, Hkv, scale, window, status);
   return launch_status();
 }
 
@@ -304,28 +456,25 @@ static int attn_f32_go(const float* q, const float* k_pages, const float* v_page
                        int* status, cudaStream_t stream) {
   const int G = Hq / Hkv;
   if (max_chunks > 0) {
-    const int code = attn_f32_launch<D, 1, true>(dim3(max_chunks, Hkv, num_seqs), q, k_pages, v_pages, out, partial, q_start,
-                                                 kv_len, block_table, table_stride, page_size, num_pages, Hq, Hkv, scale,
-                                                 window, max_chunks, status, stream);
-    if (code) return code;
-    q3::launch(attn_f32_fold_kernel<D>, dim3(Hq, num_seqs), dim3(D), 0, stream, partial, out, q_start, kv_len, Hq, window,
-               max_chunks, status);
-    return launch_status();
+#define Q3_AF_CHUNKS(G_)                                                                                                    \
+  return attn_f32_chunks<D, G_>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride, page_size,    \
+                                num_pages, num_seqs, Hq, Hkv, scale, window, max_chunks, status, stream)
+    if (G == 1) Q3_AF_CHUNKS(1);
+    if (G == 2) Q3_AF_CHUNKS(2);
+    if (G == 4) Q3_AF_CHUNKS(4);
+    Q3_AF_CHUNKS(8);
+#undef Q3_AF_CHUNKS
   }
-  if (max_q_len * G <= 8)
-    return attn_f32_launch<D, 1, false>(dim3(1, Hkv, num_seqs), q, k_pages, v_pages, out, nullptr, q_start, kv_len,
-                                        block_table, table_stride, page_size, num_pages, Hq, Hkv, scale, window, 0, status,
-                                        stream);
-#define Q3_AF_WHOLE(RPT)                                                                                                   \
-  return attn_f32_launch<D, RPT, false>(dim3((max_q_len + 8 * RPT / G - 1) / (8 * RPT / G), Hkv, num_seqs), q, k_pages,     \
-                                        v_pages, out, nullptr, q_start, kv_len, block_table, table_stride, page_size,       \
-                                        num_pages, Hq, Hkv, scale, window, 0, status, stream)
+#define Q3_AF_WALK(RPT)                                                                                                     \
+  return attn_f32_walk<D, RPT>(q, k_pages, v_pages, out, q_start, kv_len, block_table, table_stride, page_size, num_pages,   \
+                               num_seqs, max_q_len, Hq, Hkv, scale, window, status, stream)
+  if (max_q_len * G <= 8) Q3_AF_WALK(1);
   // 16 rows per block where blocks of 32 would leave SMs without one (37 tokens over 1,000 keys: 143 against 184 us), else
   // 32 (prompts of 203 and 310 tokens: 76 us against 90 with 16 rows, and 111 with 64, whose one warp per scheduler waits
   // for every shared-memory read)
-  if ((long long)((max_q_len + 32 / G - 1) / (32 / G)) * Hkv * num_seqs < sm_count()) Q3_AF_WHOLE(2);
-  Q3_AF_WHOLE(4);
-#undef Q3_AF_WHOLE
+  if ((long long)((max_q_len + 32 / G - 1) / (32 / G)) * Hkv * num_seqs < sm_count()) Q3_AF_WALK(2);
+  Q3_AF_WALK(4);
+#undef Q3_AF_WALK
 }
 
 }  // namespace q3
