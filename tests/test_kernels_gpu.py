@@ -245,6 +245,35 @@ def test_attn_f32_reports_bad_tables():
     assert int(st.item()) == 4
 
 
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("nb,rows,bw", [(8, 512, 256), (3, 16, 8), (5, 48, 136), (2, 24, 40), (2, 32, 12)])
+def test_block_diag(T, nb, rows, bw):
+    """A few tokens through the few-rows product where it takes the sizes, else a warp per row (or the library)."""
+    g = torch.Generator().manual_seed(6)
+    u = torch.randn(T, nb * bw, generator=g).to(torch.bfloat16)
+    w = torch.randn(nb, rows, bw, generator=g).to(torch.bfloat16)
+    out = torch.full((nb, T, rows), float("nan"), device="cuda")
+    ops().block_diag(dev(u), dev(w), out)
+    want = torch.einsum("tbe,bre->btr", u.double().view(T, nb, bw), w.double())
+    close(out, want, "float32", scale=float(want.abs().max()), tol=f32_accumulation_tol(bw))
+
+
+@pytest.mark.parametrize("rows,H", [(1, 2048), (8, 4), (148, 1028), (149, 2048), (9, 4096), (3, 4100)])
+@pytest.mark.parametrize("with_delta,with_out", [(True, True), (False, False)])
+def test_scale_add_rmsnorm_rows(rows, H, with_delta, with_out):
+    """bfloat16: a block per row up to one row per SM and widths of 4,096, other forms beyond."""
+    g = torch.Generator().manual_seed(8)
+    resid, w = torch.randn(rows, H, generator=g), 1 + 0.1 * torch.randn(H, generator=g)
+    delta = torch.randn(rows, H, generator=g).to(torch.bfloat16) if with_delta else None
+    r, out = dev(resid), torch.full((rows, H), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops().scale_add_rmsnorm(r, None if delta is None else dev(delta), dev(w), out if with_out else None, 1.7, 1e-6)
+    total = 1.7 * resid.double() + (0 if delta is None else delta.double())
+    want = plain.rms_norm(total, w.double(), 1e-6)
+    close(r, want, "float32")
+    if with_out:
+        close(out, want, "bfloat16")
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 def test_swiglu(dtype):
     g = torch.Generator().manual_seed(4)
