@@ -450,6 +450,42 @@ def replay(folder, dtype, seqs, schedule, **session_args):
     return r.result()
 
 
+@pytest.mark.parametrize("H,dn,rot,dims", [(16, 128, 64, 64), (3, 8, 24, 16), (5, 24, 16, 16), (2, 128, 64, 32), (2, 12, 16, 8)])
+@pytest.mark.parametrize("pairing", ["halves", "neighbours"])
+def test_latent_query_rotation_in_bfloat16(H, dn, rot, dims, pairing):
+    """Rows in pieces of eight values (and sizes that do not fit them) against the float32 kernel on the same values:
+    one rounding of the result."""
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(dims + H)
+    T = 9
+    q = torch.randn(T, H * (dn + rot), generator=g).to(torch.bfloat16).cuda()
+    freq = torch.rand(dims // 2, generator=g).cuda()
+    pos = torch.arange(100, 100 + T, dtype=torch.int32, device="cuda")
+    outs = []
+    for t in (q, q.float()):
+        plain_q, rot_q = torch.empty(T, H * dn, dtype=t.dtype, device="cuda"), torch.empty(T, H, rot, dtype=t.dtype, device="cuda")
+        ops.latent_q_post(t, H, dn, rot, dims, freq, 1.3, pos, plain_q, rot_q, pairing=pairing)
+        outs.append((plain_q, rot_q))
+    assert torch.equal(outs[0][0].float(), outs[1][0])
+    want = outs[1][1]
+    assert bool(((outs[0][1].float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("T,I,parts", [(3, 4096, 8), (9, 1024, 1), (2, 1056, 1), (5, 48, 2), (7, 40, 4)])
+def test_gated_group_norm_in_bfloat16(T, I, parts):
+    """A warp per part up to 1,024 values in multiples of eight, a block per part for the rest, against float64."""
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(I + parts)
+    y, w = torch.randn(T, I, generator=g).cuda(), (1 + 0.1 * torch.randn(I, generator=g)).cuda()
+    z = torch.randn(T, I + 16, generator=g).to(torch.bfloat16).cuda()
+    out = torch.empty(T, I, dtype=torch.bfloat16, device="cuda")
+    ops.gated_group_norm(y, z, 8, w, out, parts, 1e-5)
+    v = y.double() * torch.nn.functional.silu(z[:, 8:8 + I].double())
+    v = v.view(T, parts, -1)
+    want = (v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt()).view(T, I) * w.double()
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+
+
 @pytest.mark.parametrize("H,rank,page,gated,sink,pitch", [(3, 64, 16, True, False, 512), (2, 512, 8, False, True, 300),
                                                           (17, 128, 16, True, True, 1024)])
 def test_latent_attention_over_formed_keys(H, rank, page, gated, sink, pitch):
