@@ -116,13 +116,13 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
   const float rate = -expf(A_log[h]), db = dt_bias[h], dskip = Dp[h];
   const int x_col = h * P + p0, b_col = inner + g * N + n0, c_col = inner + G * N + g * N + n0;
   float log_total = 0.f;
-  if constexpr (VEC && PP == 4) {
+  if constexpr (VEC) {
     // Four tokens' inputs are asked for together, so that a portion pays one trip to memory per four tokens and not one
     // per token (64 heads of 64, a state of 128: 1.8 us a token before, 0.8 us now).  The arithmetic is the loop's below.
     constexpr int U = 4;
     for (int tg = t0; tg < t1; tg += U) {
       uint4 Br[U][2], Cr[U][2];
-      uint2 xr[U];
+      T xr[U][PP];
       float pre4[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -135,7 +135,12 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
           Cr[u][0] = mine_live ? reinterpret_cast<const uint4*>(row + c_col)[0] : make_uint4(0, 0, 0, 0);
           Cr[u][1] = mine_live ? reinterpret_cast<const uint4*>(row + c_col)[1] : make_uint4(0, 0, 0, 0);
         }
-        xr[u] = *reinterpret_cast<const uint2*>(row + x_col);
+        if constexpr (PP == 4) {
+          *reinterpret_cast<uint2*>(xr[u]) = *reinterpret_cast<const uint2*>(row + x_col);
+        } else {
+#pragma unroll
+          for (int c = 0; c < PP; ++c) xr[u][c] = row[x_col + c];
+        }
         pre4[u] = to_float(proj[(size_t)t * ld_proj + dt_col + h]) + db;
       }
 #pragma unroll
@@ -146,11 +151,9 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
         log_total += log_a;
         const uint32_t bw[8] = {Br[u][0].x, Br[u][0].y, Br[u][0].z, Br[u][0].w, Br[u][1].x, Br[u][1].y, Br[u][1].z, Br[u][1].w};
         const uint32_t cw[8] = {Cr[u][0].x, Cr[u][0].y, Cr[u][0].z, Cr[u][0].w, Cr[u][1].x, Cr[u][1].y, Cr[u][1].z, Cr[u][1].w};
-        const float x[4] = {__uint_as_float(xr[u].x << 16), __uint_as_float(xr[u].x & 0xffff0000u),
-                            __uint_as_float(xr[u].y << 16), __uint_as_float(xr[u].y & 0xffff0000u)};
 #pragma unroll
         for (int c = 0; c < PP; ++c) {
-          const float sx = step * x[c];
+          const float xc = to_float(xr[u][c]), sx = step * xc;
           float part = 0.f;
 #pragma unroll
           for (int i = 0; i < SSD_PER; ++i) {
@@ -160,7 +163,7 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
           }
           if (MODE != 1) {
             for (int o = L >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-            if (live && l == 0) y[(size_t)(tg + u) * inner + x_col + c] = fmaf(dskip, x[c], part);
+            if (live && l == 0) y[(size_t)(tg + u) * inner + x_col + c] = fmaf(dskip, xc, part);
           }
         }
       }
@@ -408,8 +411,13 @@ extern "C" int q3_ssd_scan(const void* xbc, int ld, const void* proj, int ld_pro
   return q3::ssd_launch<bf16, PP, VEC>(xbc, ld, proj, ld_proj, dt_col, dt_bias, A_log, Dp, state, scratch, q_start,      \
                                        slot_ids, y, B, max_q_len, H, P, N, G, num_slots, status, stream);
   if (P % 4 == 0) {
-    if (vec) { Q3_SSD(4, true) }
-    Q3_SSD(4, false)
+    // four channels per group of lanes share the reads of B and C; one where the walk of whole portions would leave most SMs
+    // without a block (one request of 64 heads of 64: 64 blocks with four, 256 with one)
+    int lanes = 1;
+    while (lanes * q3::SSD_PER < N) lanes <<= 1;
+    const bool few = !scratch && max_q_len > 1 && (long long)B * H * (P / 4) * lanes / 128 < q3::sm_count();
+    if (vec && !few) { Q3_SSD(4, true) }
+    if (!vec) { Q3_SSD(4, false) }
   }
   if (vec) { Q3_SSD(1, true) }
   Q3_SSD(1, false)
