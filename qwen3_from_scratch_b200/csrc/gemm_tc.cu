@@ -306,11 +306,26 @@ __device__ __forceinline__ void qkv_tile_epilogue(uint32_t tmem_acc, unsigned ch
 
 // Stores 32 consecutive columns of one row.  EPI 0: as they are.  EPI 1: SwiGLU on column blocks
 // (gate 8, up 8, ...), 16 outputs at half the column index.  EPI 3: the same with a ReLU gate.  EPI 4: with the gate
-// that `e` names, behind a bias.
+// that `e` names, behind a bias.  EPI 5: as they are, through the activation that `e` names (a feed-forward without a gate).
 template <int EPI, typename OutT>
 __device__ __forceinline__ void tc_store_chunk(const uint32_t (&v)[32], OutT* __restrict__ C, int row, int col0, int N,
                                                int ldc, const QkvEpilogue& e) {
-  if (EPI == 0) {
+  if (EPI == 5) {
+    // fast exponential and division as in the gates below: their error (about 2^-21) is far below the bfloat16 rounding
+    uint32_t a[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      float z = __uint_as_float(v[j]);
+      if (e.gate_act == Q3_ACT_GELU_TANH)  // (1 + tanh(y)) / 2 = sigmoid(2 y)
+        z = __fdividef(z, 1.0f + __expf(-1.5957691216057308f * fmaf(0.044715f * z, z, 1.0f) * z));
+      else if (e.gate_act == Q3_ACT_SILU)
+        z = __fdividef(z, 1.0f + __expf(-z));
+      else
+        z = fmaxf(z, 0.f) * (e.gate_act == Q3_ACT_RELU_SQ ? fmaxf(z, 0.f) : 1.0f);
+      a[j] = __float_as_uint(z);
+    }
+    tc_store_chunk<0, OutT>(a, C, row, col0, N, ldc, e);
+  } else if (EPI == 0) {
     OutT* dst = C + (size_t)row * ldc + col0;
     if (col0 + 32 <= N && ((uintptr_t)dst & 15) == 0) {
       // the thread's 32 values are contiguous in its row: 16-byte stores
@@ -906,6 +921,19 @@ extern "C" int q3_gemm_tc_gated(const void* A, const void* W, void* C, int M, in
   using bf16 = __nv_bfloat16;
   if (pair) return q3::gemm_tc_pair_launch<4, bf16>(A, W, C, M, N, K, ldc, status, stream, e);
   return q3::gemm_tc_dispatch<4, bf16>(A, W, C, M, N, K, ldc, status, stream, e);
+}
+
+// C[M, N] = act(A[M, K] * W[N, K]^T), bfloat16, by pairs of CTAs: a feed-forward without a gate, whose activation sees the
+// float32 product.  act: Q3_ACT_SILU, Q3_ACT_RELU, Q3_ACT_GELU_TANH or Q3_ACT_RELU_SQ.
+extern "C" int q3_gemm_tc_act(const void* A, const void* W, void* C, int M, int N, int K, int ldc, int act, int* status,
+                              cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || K % 8 || (act != Q3_ACT_SILU && act != Q3_ACT_RELU && act != Q3_ACT_GELU_TANH && act != Q3_ACT_RELU_SQ))
+    return Q3_ERR_SIZE;
+  if ((uintptr_t)A % 16 || (uintptr_t)W % 16) return Q3_ERR_ALIGN;
+  q3::QkvEpilogue e{};
+  e.gate_act = act;
+  return q3::gemm_tc_pair_launch<5, __nv_bfloat16>(A, W, C, M, N, K, ldc, status, stream, e);
 }
 
 // For the tests of the give-up path: see set_wait_test in tc_common.cuh.

@@ -56,6 +56,7 @@ _SIGNATURES = {
                     _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
                     _c_void_p, _c_void_p],
     "q3_gemm_skinny_block_diag": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
+    "q3_gemm_tc_act": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "q3_latent_gather": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                          _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "q3_latent_attn_tc": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
@@ -839,6 +840,29 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.T
                  1 if out.dtype == torch.float32 else 0, GEMM_TC_GATES[activation] if swiglu_blocks else 0,
                  status.data_ptr(), _stream())
     _done("gemm_tc", code, f"M {M} N {N} K {K}{' pair' if pair else ''}")
+
+
+GEMM_TC_ACTIVATIONS = ("silu", "relu", "gelu_tanh", "relu_sq")
+
+
+def gemm_tc_act_pays(rows: int, weight: torch.Tensor) -> bool:
+    """Whether the tcgen05 product with an activation in its epilogue beats the library's product and a pass over its
+    result: where the gated product runs by pairs of CTAs, at the library's rate (see ``gemm_tc_swiglu_pays`` for the lines).
+    The pass costs 13 us at 2,048 rows of 6,144; 12 such layers in a prompt step 4.15 ms with it, 4.08 without."""
+    return gemm_tc_swiglu_pays(rows, weight) == "pair"
+
+
+def gemm_tc_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, activation: str, status: torch.Tensor) -> None:
+    """out[M, N] = activation(x[M, K] @ w[N, K]^T), bfloat16, the activation applied to the float32 product."""
+    for name, t in (("x", x), ("w", w), ("out", out)):
+        _check(f"gemm_tc_act.{name}", t, torch.bfloat16)
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or tuple(out.shape) != (M, N) or activation not in GEMM_TC_ACTIVATIONS:
+        raise KernelError(f"gemm_tc_act: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, {activation}")
+    code = library().q3_gemm_tc_act(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, N, activation_code(activation, gate=True),
+                                    status.data_ptr(), _stream())
+    _done("gemm_tc_act", code, f"M {M} N {N} K {K}, {activation}")
 
 
 # ------------------------------------------------------------------ fast bfloat16 attention

@@ -153,6 +153,13 @@ class DenseMLP(FeedForward):
             h = self.up._buffer("_out", rows, self.up.out_dtype)
             ops.gemm_skinny(x, self.up.weight, h, plain_activation=self.activation)
             return self.down(h)
+        if (self.rt.dtype == torch.bfloat16 and not self.up.full_precision and x.dtype == torch.bfloat16
+                and self.activation in ops.GEMM_TC_ACTIVATIONS and ops.gemm_tc_act_pays(rows, self.up.weight)
+                and ops.gemm_tc_takes(x, self.up.weight)):
+            # prompt portions: the activation in the product's epilogue
+            h = self.up._buffer("_out", rows, self.up.out_dtype)
+            ops.gemm_tc_act(x, self.up.weight, h, self.activation, self.rt.status)
+            return self.down(h)
         h = self.up(x)
         ops.act(h, h, self.activation)
         return self.down(h)

@@ -245,6 +245,21 @@ def test_attn_f32_reports_bad_tables():
     assert int(st.item()) == 4
 
 
+@pytest.mark.parametrize("M,N,K", [(600, 1000, 328), (257, 264, 64), (1, 48, 8), (1024, 2048, 512)])
+@pytest.mark.parametrize("activation", ["silu", "relu", "gelu_tanh", "relu_sq"])
+def test_gemm_tc_with_an_activation(M, N, K, activation):
+    """The activation of the float32 product, rounded once; ragged last tiles in rows, columns and the reduction."""
+    g = torch.Generator().manual_seed(9)
+    x, w = torch.randn(M, K, generator=g).to(torch.bfloat16), (torch.randn(N, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    out, st = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16), status()
+    ops().gemm_tc_act(dev(x), dev(w), out, activation, st)
+    z = x.double() @ w.double().t()
+    f = torch.nn.functional
+    want = {"silu": f.silu(z), "relu": z.relu(), "gelu_tanh": f.gelu(z, approximate="tanh"), "relu_sq": z.relu() ** 2}[activation]
+    assert int(st.item()) == 0
+    close(out, want, "bfloat16")
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 16, 17])
 @pytest.mark.parametrize("nb,rows,bw", [(8, 512, 256), (3, 16, 8), (5, 48, 136), (2, 24, 40), (2, 32, 12)])
 def test_block_diag(T, nb, rows, bw):
