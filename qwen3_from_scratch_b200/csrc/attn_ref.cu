@@ -3,8 +3,8 @@
 // denominator (float32 throughout; probabilities are never rounded).  A query's
 // result depends only on its own keys and their order, not on how the batch was
 // cut, so the 32-bit path gives the same bits for whole prompts, portions and
-// single decoded tokens.  It serves the float32 path, sizes the fast bfloat16
-// kernels refuse, and the tests as the on-device oracle of those kernels.
+// single decoded tokens.  It serves the sizes that the other kernels (attn_f32.cu for
+// float32, the bfloat16 ones) refuse, and the tests as the on-device oracle of those kernels.
 //
 // Reference formulas (models/attn.py:402-499, kernels/triton/paged_attn.py:89-181):
 //   query at absolute position p = kv_len - q_len + i sees keys n <= p

@@ -6,7 +6,7 @@
 // W_uv c can be formed.  With 16 heads of 128 + 64 over a latent of 512 the absorbed form costs 1,088 multiply-adds per
 // query, head and key, the formed one 320, and forming 131,072 per head and key, which a portion pays once for all its
 // tokens.  At 2,048 tokens a layer's attention took 525 us absorbed (on mma.sync, with 25 us for the products around it); now
-// 32 us of attention (670 TFLOP/s), 11 us for forming keys and values and 9 us for the gather.
+// 32 us of attention (670 TFLOP/s), 11 us for forming keys and values and 3 us for the gather.
 //   latent_gather_kernel     brings a request's latents and rotated parts out of their pages into rows of their own
 //   (a library product)      keys and values of all heads, [rows, H 128 | H 128]
 //   latent_attn_tc_kernel    causal attention of one head's 128 query rows over the formed keys: scores over 128 + 64

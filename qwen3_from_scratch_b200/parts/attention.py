@@ -252,9 +252,10 @@ class LatentAttention(Mixer):
     ``pairing``: which values of a rotated part turn together, "halves" (i with i + dims / 2) or "neighbours" (2i with
     2i + 1); the frequencies are the position part's either way.
 
-    Per token the cache holds only c (plane ``c``) and r (plane ``r``), one "head" each.  Keys and values are never
-    formed: the plain query is taken through W_uk once (q' = W_uk,head^T q_plain, ``kv_rank`` values), the kernels
-    attend over the latents themselves, and the result goes through W_uv,head afterwards.  ``scale`` is used as given.
+    Per token the cache holds only c (plane ``c``) and r (plane ``r``), one "head" each.  Single tokens never form keys and
+    values: the plain query is taken through W_uk once (q' = W_uk,head^T q_plain, ``kv_rank`` values), the kernels attend
+    over the latents themselves, and the result goes through W_uv,head afterwards.  Steps of prompt portions form every
+    head's keys and values from the latents first where the kernels take the sizes.  ``scale`` is used as given.
     Norms, angles, scores, weights and the gate are float32 in every run.  ``position``: a part with
     ``frequencies()`` (``rotary_stretched``); ``names``: the tensors' names after the part's own."""
 
