@@ -164,6 +164,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 // rows of A come through L1, which the block's warps share.  The chains' sums meet in shared memory.
 constexpr int GFS_WARPS = 8;
 constexpr int GFS_MAX_ROWS = 16;
+constexpr int GFS_MAX_SEGS = 16;  // K up to 16,384; times the groups of a block never more than this, whatever K
 
 __device__ __forceinline__ void gf_load8(float (&v)[8], const float* p) {  // read once: not kept in L1
   asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -274,9 +275,13 @@ static int gemm_f32_rows_launch(const float* A, const float* W, float* C, int M,
                                 int segs, int seg_warps, cudaStream_t stream) {
   const int groups = GFS_WARPS / seg_warps;
   const size_t smem = (size_t)groups * R * MT * segs * 32 * sizeof(float);
+  // The limit is the function's, for all threads: always set to the most that any K asks for, so that no call lowers it
+  // under another's launch.
+  constexpr size_t most = (size_t)R * MT * GFS_MAX_SEGS * 32 * sizeof(float);
+  if (smem > most) return Q3_ERR_SIZE;
   auto kernel = gemm_f32_rows_kernel<MT, R>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (most > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return (int)e;
   }
   q3::launch(kernel, dim3((N + groups * R - 1) / (groups * R)), dim3(GFS_WARPS * 32), smem, stream, A, W, C, M, N, K, lda, ldw,
@@ -294,7 +299,7 @@ extern "C" int q3_gemm_f32_nt(const float* A, const float* W, float* C, int M, i
   if (K <= 0) return Q3_ERR_SIZE;
   const int segs = (K + GF_SEG - 1) / GF_SEG;
   // Up to 16 rows stream W once; the sums of up to 16 segments (K = 16,384) fit the block's shared memory.
-  if (M <= GFS_MAX_ROWS && segs <= 16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && (uintptr_t)A % 32 == 0 &&
+  if (M <= GFS_MAX_ROWS && segs <= GFS_MAX_SEGS && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && (uintptr_t)A % 32 == 0 &&
       (uintptr_t)W % 32 == 0) {
     const int seg_warps = segs < GFS_WARPS ? segs : GFS_WARPS;
     const int groups = GFS_WARPS / seg_warps;

@@ -185,6 +185,38 @@ def test_gemm_f32_orders_agree(N, K):
         assert torch.equal(wide[:, :N], out[:M]) and bool(torch.isnan(wide[:, N:]).all()), M
 
 
+def test_gemm_f32_of_different_lengths_from_several_threads():
+    """Threads with streams of their own run the few-rows kernel at lengths of K that need different amounts of shared
+    memory: no launch is refused because another thread has just set a smaller limit.  The threads call the library
+    itself, so that they spend their time inside its launches."""
+    import threading
+    g = torch.Generator().manual_seed(6)
+    M, N, calls = 16, 1024, 15000
+    jobs, refused = [], []
+    for K in (12288, 4096, 12288, 4096):
+        a, w = dev(torch.randn(M, K, generator=g)), dev(torch.randn(N, K, generator=g))
+        out, want = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+        ops().gemm_f32_nt(a, w, want)
+        jobs.append((a, w, out, want, K, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    launch = ops().library()._lib.q3_gemm_f32_nt
+
+    def work(job):
+        a, w, out, _, K, stream = job
+        args = (a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, N, stream.cuda_stream)
+        refused.append(sum(launch(*args) != 0 for _ in range(calls)))
+
+    threads = [threading.Thread(target=work, args=(job,)) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert refused == [0] * len(jobs)
+    for _, _, out, want, _, _ in jobs:
+        assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("hq,hkv,d,page_size,window", [(16, 8, 128, 16, None), (8, 1, 64, 8, None), (4, 4, 128, 16, 70),
                                                        (8, 2, 64, 32, 1)])
 def test_attn_f32(hq, hkv, d, page_size, window):
