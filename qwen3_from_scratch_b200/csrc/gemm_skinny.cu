@@ -49,8 +49,7 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 }
 
 // NT: token tiles of 8 (1 or 2).  WK: warps that share a group of 16 features and split K.
-// EPI: 0 store, 1 SwiGLU on alternating blocks of eight rows, 2 added into the float32 stream, 3 a block-diagonal
-// product's store (a form of its own: what it asks on the way cost every plain product of a decode step 45 ns).
+// EPI: 0 store, 1 SwiGLU on alternating blocks of eight rows, 2 added into the float32 stream.
 // (The kernel is asked to fit three blocks per SM where K is not split in the block, which is the long
 // stream of the output head, and with two token tiles: there, left to itself, the compiler used fewer registers
 // than three blocks allow and took the loads one after the other.  Two token tiles are short of registers at
@@ -75,8 +74,6 @@ struct SkinnyFuse {
   float limit;          // EPI 1: of Q3_ACT_LIMITED
   int x_rows;           // 0, or: the features in groups of so many (a multiple of 16), group i reads the i-th of several X
   long long x_stride;   // values from one X to the next
-  int x_ld;             // EPI 3: values from one row of X to the next
-  long long out_stride; // EPI 3: values of `out` from one group's results to the next
 };
 
 constexpr int GS_SS_ROWS = 16;  // row pitch of the partial sums
@@ -164,7 +161,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __r
   for (int i = 0; i < NT; ++i) {
     const int tok = i * 8 + gid;
     x_ok[i] = tok < T;
-    x_row[i] = X + (size_t)(x_ok[i] ? tok : 0) * (EPI == 3 ? fuse.x_ld : K) + 8 * tid4;
+    x_row[i] = X + (size_t)(x_ok[i] ? tok : 0) * K + 8 * tid4;
     if (fuse.x_rows && active) x_row[i] += (row0 / fuse.x_rows) * fuse.x_stride;
   }
   auto multiply = [&](int g0, const uint4 (&lo)[GS_UNROLL], const uint4 (&hi)[GS_UNROLL]) {
@@ -222,9 +219,8 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __r
   }
   __syncthreads();
   if (ksplit != 0 || !active) return;
-  if (EPI == 0 || EPI == 3) {
+  if (EPI == 0) {
     // 16 features x T tokens; consecutive lanes take consecutive features of one token
-    OutT* dst = EPI == 3 ? out + (row0 / fuse.x_rows) * (fuse.out_stride - fuse.x_rows) : out;
     for (int e = lane; e < 16 * 8 * NT; e += 32) {
       const int f = e & 15, tok = e >> 4;
       if (tok >= T || row0 + f >= N) continue;
@@ -233,7 +229,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __r
       for (int s = 0; s < WK; ++s) v += red[warp + s][f][tok];
       if (NORMED) v *= rs_s[tok];
       if (fuse.plain_act) v = activate(v, fuse.plain_act - 1);
-      dst[(size_t)tok * ldo + row0 + f] = from_float<OutT>(v);
+      out[(size_t)tok * ldo + row0 + f] = from_float<OutT>(v);
     }
   } else if (EPI == 2) {
     // added into the stream; the 16 lanes that share a row leave the sum of squares of their new values
@@ -403,23 +399,6 @@ extern "C" int q3_gemm_skinny_groups(const void* X, const void* W, void* out, in
   fuse.x_stride = (long long)T * K;
   if (T <= 8) return q3::gemm_skinny_launch<1, 0, bf16>(X, W, out, T, N, K, ldo, stream, fuse);
   return q3::gemm_skinny_launch<2, 0, bf16>(X, W, out, T, N, K, ldo, stream, fuse);
-}
-
-// A block-diagonal product: group i of `group` features reads the i-th run of K values of the rows of X ([T, N / group * K])
-// and leaves float32 [T, group] at out + i * T * group.  T <= 16, bfloat16 in, group a multiple of 16.
-extern "C" int q3_gemm_skinny_block_diag(const void* X, const void* W, float* out, int T, int N, int K, int group,
-                                         cudaStream_t stream) {
-  if (T <= 0 || N <= 0) return 0;
-  if (T > 16 || K <= 0 || K % 8 || group <= 0 || group % 16 || N % group || (long long)N / group * K > 0x7fffffffll)
-    return Q3_ERR_SIZE;
-  if ((uintptr_t)X % 16 || (uintptr_t)W % 16) return Q3_ERR_ALIGN;
-  q3::SkinnyFuse fuse{};
-  fuse.x_rows = group;
-  fuse.x_stride = K;
-  fuse.x_ld = N / group * K;
-  fuse.out_stride = (long long)T * group;
-  if (T <= 8) return q3::gemm_skinny_launch<1, 3, float>(X, W, out, T, N, K, group, stream, fuse);
-  return q3::gemm_skinny_launch<2, 3, float>(X, W, out, T, N, K, group, stream, fuse);
 }
 
 // The forms that take the norm kernels out of a decode step (see the head of the file), T <= 16.

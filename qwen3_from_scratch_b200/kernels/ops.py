@@ -55,7 +55,6 @@ _SIGNATURES = {
     "q3_attn_ref": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                     _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
                     _c_void_p, _c_void_p],
-    "q3_gemm_skinny_block_diag": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "q3_gemm_tc_act": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "q3_latent_gather": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                          _c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -1343,14 +1342,6 @@ def block_diag(u: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None
         raise KernelError(f"block_diag: u {tuple(u.shape)}, weight {tuple(weight.shape)}, out {tuple(out.shape)}")
     if u.dtype == torch.bfloat16 and T > BLOCK_DIAG_FEW_ROWS:
         torch.bmm(u.view(T, nb, bw).transpose(0, 1), weight.transpose(1, 2), out_dtype=torch.float32, out=out)
-        return
-    if (u.dtype == torch.bfloat16 and T <= SKINNY_MAX_ROWS and bw % 8 == 0 and rows % 16 == 0 and u.data_ptr() % 16 == 0
-            and weight.data_ptr() % 16 == 0):
-        # the few-rows product, whose tensor-core tiles take all tokens at once (8 blocks of 256 x 512 and 8 tokens: 3.8 us;
-        # 15.7 us with a warp per row walking over the tokens)
-        code = library().q3_gemm_skinny_block_diag(u.data_ptr(), weight.data_ptr(), out.data_ptr(), T, nb * rows, bw, rows,
-                                                   _stream())
-        _done("gemm_skinny_block_diag", code, f"T {T}, {nb} blocks of {rows} x {bw}")
         return
     code = library().q3_block_diag(u.data_ptr(), weight.data_ptr(), out.data_ptr(), dtype_tag(u.dtype), T, nb, bw, rows,
                                    _stream())

@@ -305,6 +305,25 @@ def test_block_diag(T, nb, rows, bw):
     close(out, want, "float32", scale=float(want.abs().max()), tol=f32_accumulation_tol(bw))
 
 
+@pytest.mark.parametrize("T", [1, 2, 3, 8, 16])
+@pytest.mark.parametrize("nb,rows,bw", [(8, 512, 256), (3, 17, 8), (2, 40, 136), (1, 33, 1024), (2, 16, 1032), (2, 24, 12)])
+def test_block_diag_of_a_few_tokens_keeps_its_bits(T, nb, rows, bw):
+    """The kernel for a few tokens adds in the order of the plain one, which takes rows that are not 16-byte aligned:
+    the same bits, and no further from 64 bits than one rounding per addition of the longest chain."""
+    g = torch.Generator().manual_seed(7)
+    u = torch.randn(T, nb * bw, generator=g).to(torch.bfloat16)
+    w = torch.randn(nb, rows, bw, generator=g).to(torch.bfloat16)
+    out, want = (torch.full((nb, T, rows), float("nan"), device="cuda") for _ in range(2))
+    ops().block_diag(dev(u), dev(w), out)
+    shifted = torch.empty(T * nb * bw + 1, device="cuda", dtype=torch.bfloat16)[1:].view(T, nb * bw)
+    ops().block_diag(shifted.copy_(u), dev(w), want)
+    assert torch.equal(out, want)
+    exact = torch.einsum("tbe,bre->btr", u.double().view(T, nb, bw), w.double())
+    steps = -(-bw // 32) + 5
+    bound = steps * 2.0 ** -24 * torch.einsum("tbe,bre->btr", u.double().abs().view(T, nb, bw), w.double().abs())
+    assert bool(((out.cpu().double() - exact).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("rows,H", [(1, 2048), (8, 4), (148, 1028), (149, 2048), (9, 4096), (3, 4100)])
 @pytest.mark.parametrize("with_delta,with_out", [(True, True), (False, False)])
 def test_scale_add_rmsnorm_rows(rows, H, with_delta, with_out):
