@@ -64,17 +64,26 @@ __device__ __forceinline__ void load_chunk(const __nv_bfloat16* __restrict__ xbc
     cum_s[t] = rate * step;  // the log-decay, summed below
   }
   __syncthreads();
-  if (threadIdx.x < 32) {  // a scan over the 64 tokens, two per lane
-    const float a = cum_s[2 * threadIdx.x], both = a + cum_s[2 * threadIdx.x + 1];
-    float run = both;
+  if (threadIdx.x == 0) {
+    // 64 additions in the order of the tokens: the difference of two sums, which is all that is used, then has the rounding
+    // errors of the steps between them only.  (A tree of shuffles left each sum its own: the states of 300 tokens were 1.25
+    // times further from 64 bits.)  Sixteen values are read together, so that the chain waits for additions, not for loads.
+    float4* c4 = reinterpret_cast<float4*>(cum_s);
+    float run = 0.f;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float below = __shfl_up_sync(0xffffffffu, run, o);
-      if ((int)threadIdx.x >= o) run += below;
+    for (int t = 0; t < SM_Q / 4; t += 4) {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = c4[t + i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i].x = run += v[i].x;
+        v[i].y = run += v[i].y;
+        v[i].z = run += v[i].z;
+        v[i].w = run += v[i].w;
+        c4[t + i] = v[i];
+      }
     }
-    const float before = __shfl_up_sync(0xffffffffu, run, 1);
-    cum_s[2 * threadIdx.x] = threadIdx.x ? before + a : a;
-    cum_s[2 * threadIdx.x + 1] = run;
   }
   __syncthreads();
 }
