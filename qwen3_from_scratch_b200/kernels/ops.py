@@ -60,7 +60,6 @@ _SIGNATURES = {
                          _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "q3_latent_attn_tc": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
                           _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
-    "q3_latent_attn_tc_wait_test": [ctypes.c_uint, _c_int],
     "q3_attn_f32": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
                     _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void_p, _c_void_p],
     "q3_attn_decode": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
@@ -231,7 +230,7 @@ _SIGNATURES = {
 }
 
 
-_WAIT_TEST = ("q3_gemm_tc_wait_test", "q3_attn_tc_wait_test", "q3_attn_decode_tma_wait_test")
+_WAIT_TEST = ("q3_gemm_tc_wait_test", "q3_attn_tc_wait_test", "q3_attn_decode_tma_wait_test", "q3_latent_attn_tc_wait_test")
 
 
 def library() -> ctypes.CDLL:

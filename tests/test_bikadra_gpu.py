@@ -574,6 +574,41 @@ def test_latent_attention_over_formed_keys(H, rank, page, gated, sink, pitch):
     assert int(status.item()) & 4
 
 
+def test_a_wait_over_formed_keys_that_runs_out_is_given_up_cleanly():
+    """The bounded waits of the attention over formed keys, made to run out: the loader leaves out the second tile of keys.
+    The kernel returns by itself with the time-out bit set, and the next ordinary launch, which needs the tensor memory and
+    shared memory that the abandoned blocks held, gives the same bits as the one before."""
+    from types import SimpleNamespace
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(91)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    bf = lambda *s: (torch.randn(*s, generator=g) * 0.5).to(torch.bfloat16).cuda()  # noqa: E731
+    T, H, rank = 400, 3, 64  # blocks of one to four tiles of keys
+    c_pages, r_pages, table = bf(25, 1, 16, rank), bf(25, 1, 16, 64), i32([list(range(25))])
+    q_plain, q_rot, up = bf(T, H * 128), bf(T, H, 64), bf(2 * H * 128, rank)
+    c_rows, r_rows, kv, out = bf(T, rank), bf(T, 64), bf(T, 2 * H * 128), bf(T, H * 128)
+    ctx = SimpleNamespace(positions=i32([0] * T), q_start=i32([0, T]), kv_len=i32([T]), num_seqs=1, num_decode=0, max_q_len=T,
+                          max_kv_len=T)
+
+    def run():
+        status = i32([0])
+        ops.latent_attention_formed(q_plain, q_rot, c_pages, r_pages, ctx, table, up.t(), c_rows, r_rows, kv, out, 0.07, status)
+        torch.cuda.synchronize()
+        return int(status.item())
+
+    assert run() == 0
+    want = out.clone()
+    try:
+        ops.set_wait_test(limit=1 << 14, drop_copy=1)
+        word = run()
+    finally:
+        ops.set_wait_test()
+    assert word & 16, f"status {word}: the time-out bit is not set"
+    out.zero_()
+    assert run() == 0
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 @pytest.mark.parametrize("key", list(CONFIGS))
 def test_model_whole_decoded_and_in_portions(folders, key, dtype):
