@@ -62,9 +62,14 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
   const int c = t & 7, r8 = t >> 3;
   const int k_piece = (c >> 1) * GF_STEP + (c & 1) * 4;
   const uint32_t dst0 = r8 * 128 + ((c ^ r8) << 4);
-  const int segs = (K + GF_SEG - 1) / GF_SEG, items = segs * 8;
+  // Only what holds a k below K is fetched and multiplied: of the last segment's chains those that begin there, and of a
+  // chain's four pieces (j) those that do.  (K = 64: 8 of 32 chains and one piece of four in each.  What is left out would
+  // add zeros to sums that are not negative zero: the bits are the same.)
+  const int segs = (K + GF_SEG - 1) / GF_SEG, rem = K - (segs - 1) * GF_SEG - group * (8 * GF_LANE);
+  const int items = (segs - 1) * 8 + max(0, min(8, (rem + GF_LANE - 1) / GF_LANE));  // chains of this group
   auto fetch = [&](int item) {
     const int k = (item >> 3) * GF_SEG + k_piece + (group * 8 + (item & 7)) * GF_LANE;
+    if (k - (c & 1) * 4 >= K) return;  // the piece is not read
     const uint32_t dst = stages + (item % GF_STAGES) * GF_STAGE_BYTES + dst0;
 #pragma unroll
     for (int p = 0; p < 16; ++p) {
@@ -106,8 +111,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     for (int i = 0; i < 8; ++i)
 #pragma unroll
       for (int j = 0; j < 8; ++j) part[i][j] = 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    auto multiply = [&](int q) {
       float4 a[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) a[i] = gf_lds(a_row + i * 1024 + ((q ^ ty) << 4));
@@ -123,6 +127,12 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 #pragma unroll
         for (int i = 0; i < 8; ++i) part[i][j] = fmaf(a[i].w, w.w, part[i][j]);
       }
+    };
+    const int left = min(GF_SEG, K - (item >> 3) * GF_SEG - (group * 8 + (item & 7)) * GF_LANE);
+#pragma unroll 1
+    for (int q = 0; q < 8 && q * (GF_STEP / 2) < left; q += 2) {
+      multiply(q);
+      multiply(q + 1);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -153,6 +163,111 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (n0 + col + i < N) dst[i] = v[i];
+    }
+  }
+}
+
+// ---------------------------------------------------------------- short reductions
+// K up to 128, where the tiles above would leave two or three of their four groups without a chain: 64 x 64 outputs per
+// block, 4 x 4 per thread, all of K in shared memory at once, the chains one after the other (T_0, then T_1; the other two
+// are zero).  34 KB for K = 64, so that several blocks share an SM and one's copies run under another's products.  Bound by
+// shared-memory reads (eight of 16 bytes per 64 FMA) and, for the smallest K, by the stores: 2,048 x 4,096 outputs of K = 64
+// 45 us (24 TFLOP/s; the tiles above 96), of K = 128 77 us (99); the kernel before these took 53 and 99 us.
+constexpr int GFK_MAX = 128, GFK_THREADS = 256;
+
+template <bool VEC>
+__global__ void __launch_bounds__(GFK_THREADS)
+gemm_f32_short_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
+                      int lda, int ldw, int ldc, int out_vec) {
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) float gfk_smem[];  // [64 rows of A, then 64 of W][pitch]
+  const int chains = (K + GF_LANE - 1) / GF_LANE, pieces = 2 * chains, pitch = 8 * chains + 4;  // eight rows: other banks
+  const int m_tiles = (M + GF_T - 1) / GF_T;
+  const int m0 = (blockIdx.x % m_tiles) * GF_T, n0 = (blockIdx.x / m_tiles) * GF_T;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(gfk_smem);
+  for (int e = threadIdx.x; e < 2 * GF_T * pieces; e += GFK_THREADS) {
+    const int r = e / pieces, k = (e - r * pieces) * 4;
+    const bool of_a = r < GF_T;
+    const int row = of_a ? m0 + r : n0 + r - GF_T;
+    const bool in_row = row < (of_a ? M : N);
+    const float* src = of_a ? A + (size_t)min(row, M - 1) * lda : W + (size_t)min(row, N - 1) * ldw;
+    const uint32_t dst = base + (r * pitch + k) * 4;
+    if (VEC) {
+      gf_copy<16>(dst, src + (k < K ? k : 0), in_row && k < K);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) gf_copy<4>(dst + 4 * i, src + (k + i < K ? k + i : 0), in_row && k + i < K);
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // rows ty + 16 i of A, tx + 16 j of W
+  const uint32_t a_row = base + ty * pitch * 4, w_row = base + (GF_T + tx) * pitch * 4;
+  float sum[4][4], T[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[i][j] = T[i][j] = 0.f;
+#pragma unroll 2
+  for (int l = 0; l < chains; ++l) {
+    if (l == 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sum[i][j] = T[i][j];
+          T[i][j] = 0.f;
+        }
+    }
+    float part[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 a[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = gf_lds(a_row + (16 * i * pitch + 8 * l + 4 * h) * 4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 w = gf_lds(w_row + (16 * j * pitch + 8 * l + 4 * h) * 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[i][j] = fmaf(a[i].x, w.x, part[i][j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[i][j] = fmaf(a[i].y, w.y, part[i][j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[i][j] = fmaf(a[i].z, w.z, part[i][j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[i][j] = fmaf(a[i].w, w.w, part[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) T[i][j] += part[i][j];
+  }
+  // through shared memory, so that a row's values leave side by side
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) gfk_smem[(ty + 16 * i) * (GF_T + 4) + tx + 16 * j] = sum[i][j] + T[i][j];
+  __syncthreads();
+  for (int e = threadIdx.x; e < GF_T * GF_T / 4; e += GFK_THREADS) {
+    const int r = e / (GF_T / 4), col = (e % (GF_T / 4)) * 4;
+    if (m0 + r >= M || n0 + col >= N) continue;
+    const float4 v = *reinterpret_cast<const float4*>(&gfk_smem[r * (GF_T + 4) + col]);
+    float* dst = C + (size_t)(m0 + r) * ldc + n0 + col;
+    if (out_vec && n0 + col + 4 <= N) {
+      *reinterpret_cast<float4*>(dst) = v;
+    } else {
+      const float vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (n0 + col + i < N) dst[i] = vs[i];
     }
   }
 }
@@ -298,9 +413,14 @@ extern "C" int q3_gemm_f32_nt(const float* A, const float* W, float* C, int M, i
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return Q3_ERR_SIZE;
   const int segs = (K + GF_SEG - 1) / GF_SEG;
-  // Up to 16 rows stream W once; the sums of up to 16 segments (K = 16,384) fit the block's shared memory.
-  if (M <= GFS_MAX_ROWS && segs <= GFS_MAX_SEGS && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && (uintptr_t)A % 32 == 0 &&
-      (uintptr_t)W % 32 == 0) {
+  // Up to 16 rows stream W once; the sums of up to 16 segments (K = 16,384) fit the block's shared memory.  A short reduction
+  // gives a lane of that kernel little to do per row of A: there the kernels below are the faster ones (us for N = 4,096:
+  // 8 rows, K = 32 5.5 against 3.5, K = 64 5.5 and 5.6; 16 rows, K = 64 7.7 and 4.8; 16 rows of N = 150,000, K = 192 222 and 175,
+  // but 7.8 and 11.6 for N = 4,096, where the tiles are fewer than the SMs).
+  const bool streams = K >= 256 || (K > GFK_MAX && (M <= 8 || (N + GF_T - 1) / GF_T * 2 <= sm_count())) ||
+                       (K <= GFK_MAX && M <= 8 && K >= 8 * M);
+  if (streams && M <= GFS_MAX_ROWS && segs <= GFS_MAX_SEGS && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 &&
+      (uintptr_t)A % 32 == 0 && (uintptr_t)W % 32 == 0) {
     const int seg_warps = segs < GFS_WARPS ? segs : GFS_WARPS;
     const int groups = GFS_WARPS / seg_warps;
     // four weight rows per warp share the reads of A; two where four would leave SMs without a block
@@ -319,6 +439,15 @@ extern "C" int q3_gemm_f32_nt(const float* A, const float* W, float* C, int M, i
   const int out_vec = ldc % 4 == 0 && (uintptr_t)C % 16 == 0;
   const long long m_tiles = (M + GF_T - 1) / GF_T, n_tiles = (N + GF_T - 1) / GF_T;
   if (m_tiles > 65535 || m_tiles * n_tiles > 0x7fffffffll) return Q3_ERR_SIZE;
+  if (K <= GFK_MAX) {
+    constexpr int most = 2 * GF_T * (GFK_MAX + 4) * (int)sizeof(float);
+    const size_t smem = max((size_t)2 * GF_T * (8 * ((K + 7) / 8) + 4), (size_t)GF_T * (GF_T + 4)) * sizeof(float);
+    auto kernel = vec ? gemm_f32_short_kernel<true> : gemm_f32_short_kernel<false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return (int)e;
+    q3::launch(kernel, dim3((unsigned)(m_tiles * n_tiles)), dim3(GFK_THREADS), smem, stream, A, W, C, M, N, K, lda, ldw, ldc, out_vec);
+    return launch_status();
+  }
   auto kernel = vec ? gemm_f32_tile_kernel<true> : gemm_f32_tile_kernel<false>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
   if (e != cudaSuccess) return (int)e;

@@ -185,6 +185,41 @@ def test_gemm_f32_orders_agree(N, K):
         assert torch.equal(wide[:, :N], out[:M]) and bool(torch.isnan(wide[:, N:]).all()), M
 
 
+@pytest.mark.parametrize("N,K", [(70, 1), (130, 7), (64, 12), (200, 64), (65, 72), (100, 124), (64, 128), (130, 132), (9000, 136),
+                                 (70, 200), (64, 769), (130, 1030), (70, 1100)])
+def test_gemm_f32_of_short_and_ragged_reductions(N, K):
+    """All of K in one tile up to 128; beyond it the chains and pieces that lie past K are left out.  Every row has the same
+    bits whatever the number of rows, and the sums are those of float32 chains."""
+    g = torch.Generator().manual_seed(15)
+    a, w = torch.randn(130, K, generator=g), torch.randn(N, K, generator=g)
+    A, W = dev(a), dev(w)
+    out = torch.full((130, N), float("nan"), device="cuda")
+    ops().gemm_f32_nt(A, W, out)
+    want = a.double() @ w.double().t()
+    assert float((out.cpu().double() - want).abs().max()) <= 1e-6 * max(K, 8) ** 0.5 * float(want.abs().max())
+    for M in (1, 4, 5, 8, 9, 16, 17, 64):
+        wide = torch.full((M, N + 3), float("nan"), device="cuda")
+        ops().gemm_f32_nt(A[:M].contiguous(), W, wide[:, :N])
+        assert torch.equal(wide[:, :N], out[:M]) and bool(torch.isnan(wide[:, N:]).all()), M
+
+
+def test_gemm_f32_takes_less_time_for_a_shorter_reduction():
+    """A product of K = 32 moves and multiplies a thirtieth of what K = 1,024 does: it takes less than half the time (an
+    eighth is measured), which it would not if the reduction were padded to a fixed length."""
+    times = {}
+    for K in (32, 1024):
+        a, w, out = (torch.randn(n, k, device="cuda") for n, k in ((2048, K), (2048, K), (2048, 2048)))
+        events = [torch.cuda.Event(enable_timing=True) for _ in range(8)]
+        ops().gemm_f32_nt(a, w, out)
+        for e in events:
+            e.record()
+            for _ in range(4):
+                ops().gemm_f32_nt(a, w, out)
+        torch.cuda.synchronize()
+        times[K] = min(x.elapsed_time(y) for x, y in zip(events, events[1:]))
+    assert times[32] < 0.5 * times[1024], times
+
+
 def test_gemm_f32_of_different_lengths_from_several_threads():
     """Threads with streams of their own run the few-rows kernel at lengths of K that need different amounts of shared
     memory: no launch is refused because another thread has just set a smaller limit.  The threads call the library
