@@ -429,9 +429,14 @@ extern "C" int q3_gated_group_norm(const float* y, const void* z, int ld_z, int 
   if (T <= 0 || I <= 0) return 0;
   if (parts <= 0 || I % parts || parts > 65535) return Q3_ERR_SIZE;
   const int width = I / parts;
-  if (dtype == Q3_BF16 && width % 8 == 0 && width <= 32 * 8 * q3::GN_MAX_CH && z_col % 8 == 0 && ld_z % 8 == 0 &&
-      (uintptr_t)y % 16 == 0 && (uintptr_t)z % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)weight % 16 == 0) {
-    const long long units = (long long)T * parts, blocks = (units + q3::GN_WARPS - 1) / q3::GN_WARPS;
+  // A warp per part where the parts are many; few of them (decoding) are one chain of latencies each, which a whole block
+  // makes shorter (width 512: 512 parts 3.1 us with a block each, 3.2 with a warp, 8 parts 2.4 and 3.0; 2,400 parts 7.2 and
+  // 4.2.  Width 1,024: 300 parts 3.8 and 4.7).
+  const long long units = (long long)T * parts;
+  if (dtype == Q3_BF16 && units > 4 * q3::sm_count() && width % 8 == 0 && width <= 32 * 8 * q3::GN_MAX_CH && z_col % 8 == 0 &&
+      ld_z % 8 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)z % 16 == 0 && (uintptr_t)out % 16 == 0 &&
+      (uintptr_t)weight % 16 == 0) {
+    const long long blocks = (units + q3::GN_WARPS - 1) / q3::GN_WARPS;
     if (blocks > 0x7fffffffll) return Q3_ERR_SIZE;
     q3::launch(q3::gated_group_norm_warp_kernel, dim3((unsigned)blocks), dim3(q3::GN_WARPS * 32), 0, stream, y,
                (const __nv_bfloat16*)z, ld_z, z_col, weight, (__nv_bfloat16*)out, units, I, parts, eps);

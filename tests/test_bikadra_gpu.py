@@ -513,6 +513,21 @@ def test_gated_group_norm_in_bfloat16(T, I, parts):
     assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
 
 
+@pytest.mark.parametrize("T,I,parts", [(74, 512, 8), (75, 512, 8), (600, 1024, 1), (600, 1056, 1), (300, 40, 5)])
+def test_gated_group_norm_of_many_parts_in_bfloat16(T, I, parts):
+    """A block per part up to four parts for each of 148 SMs, a warp per part beyond (widths up to 1,024 in multiples of
+    eight): both against float64, one rounding of the result."""
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(I + parts)
+    y, w = torch.randn(T, I, generator=g).cuda(), (1 + 0.1 * torch.randn(I, generator=g)).cuda()
+    z = torch.randn(T, I + 16, generator=g).to(torch.bfloat16).cuda()
+    out = torch.full((T, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.gated_group_norm(y, z, 8, w, out, parts, 1e-5)
+    v = (y.double() * torch.nn.functional.silu(z[:, 8:8 + I].double())).view(T, parts, -1)
+    want = (v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt()).view(T, I) * w.double()
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+
+
 @pytest.mark.parametrize("H,rank,page,gated,sink,pitch", [(3, 64, 16, True, False, 512), (2, 512, 8, False, True, 300),
                                                           (17, 128, 16, True, True, 1024)])
 def test_latent_attention_over_formed_keys(H, rank, page, gated, sink, pitch):
