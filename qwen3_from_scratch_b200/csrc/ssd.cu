@@ -57,7 +57,8 @@ __device__ __forceinline__ void ssd_load16(const T* __restrict__ row, int col, i
 // the threads (so that a chunk's state comes and goes in 16-byte pieces of whole lines), then H decay products
 // (padded to a multiple of four):
 // `record_floats` floats; chunk j of request b is record q_start[b] / SSD_CHUNK + b + j.
-template <typename T, int PP, bool VEC, int MODE>
+// U (VEC only): tokens whose inputs are asked for together.
+template <typename T, int PP, bool VEC, int MODE, int U>
 __global__ void __launch_bounds__(128)
 ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, int ld_proj, int dt_col,
                 const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ Dp,
@@ -118,11 +119,11 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
   float log_total = 0.f;
   if constexpr (VEC) {
     // Four tokens' inputs are asked for together, so that a portion pays one trip to memory per four tokens and not one
-    // per token (64 heads of 64, a state of 128: 1.8 us a token before, 0.8 us now).  The arithmetic is the loop's below.
-    constexpr int U = 4;
+    // per token (64 heads of 64, a state of 128: 1.8 us a token before, 0.8 us now).  A step whose longest portion is shorter
+    // asks for one or two (64 single tokens: 112 us with loads of four, 90 us here).  The arithmetic is the loop's below.
     for (int tg = t0; tg < t1; tg += U) {
       uint4 Br[U][2], Cr[U][2];
-      T xr[U][PP];
+      __align__(8) T xr[U][PP];
       float pre4[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -357,20 +358,23 @@ static int ssd_launch(const void* xbc, int ld, const void* proj, int ld_proj, in
   if (blocks > 65535) return Q3_ERR_SIZE;
   const T* x = (const T*)xbc;
   const T* pr = (const T*)proj;
+  constexpr int U = VEC ? 4 : 1;
   if (!scratch) {
-    launch(ssd_scan_kernel<T, PP, VEC, 0>, dim3(B, (unsigned)blocks), dim3(128), 0, stream, x, ld, pr, ld_proj, dt_col,
-           dt_bias, A_log, Dp, state, scratch, q_start, slot_ids, y, H, P, N, G, L, num_slots, (size_t)0, status);
+    auto walk = max_q_len <= 1 ? ssd_scan_kernel<T, PP, VEC, 0, 1>
+                : max_q_len <= 3 ? ssd_scan_kernel<T, PP, VEC, 0, VEC ? 2 : 1> : ssd_scan_kernel<T, PP, VEC, 0, U>;
+    launch(walk, dim3(B, (unsigned)blocks), dim3(128), 0, stream, x, ld, pr, ld_proj, dt_col, dt_bias, A_log, Dp, state,
+           scratch, q_start, slot_ids, y, H, P, N, G, L, num_slots, (size_t)0, status);
     return launch_status();
   }
   const int chunks = (max_q_len + SSD_CHUNK - 1) / SSD_CHUNK;
   if (chunks > 65535) return Q3_ERR_SIZE;
   const size_t all = (size_t)threads * PP * SSD_PER, record_floats = all + ((H + 3) & ~3);
   if ((all + 255) / 256 > 65535 || record_floats % 4) return Q3_ERR_SIZE;
-  launch(ssd_scan_kernel<T, PP, VEC, 1>, dim3(B, (unsigned)blocks, chunks), dim3(128), 0, stream, x, ld, pr, ld_proj,
+  launch(ssd_scan_kernel<T, PP, VEC, 1, U>, dim3(B, (unsigned)blocks, chunks), dim3(128), 0, stream, x, ld, pr, ld_proj,
          dt_col, dt_bias, A_log, Dp, state, scratch, q_start, slot_ids, y, H, P, N, G, L, num_slots, record_floats, status);
   launch(ssd_carry_kernel, dim3(B, (unsigned)((all + 255) / 256)), dim3(256), 0, stream, scratch, state, q_start, slot_ids,
          H, N, P, PP, L, num_slots, record_floats);
-  launch(ssd_scan_kernel<T, PP, VEC, 2>, dim3(B, (unsigned)blocks, chunks), dim3(128), 0, stream, x, ld, pr, ld_proj,
+  launch(ssd_scan_kernel<T, PP, VEC, 2, U>, dim3(B, (unsigned)blocks, chunks), dim3(128), 0, stream, x, ld, pr, ld_proj,
          dt_col, dt_bias, A_log, Dp, state, scratch, q_start, slot_ids, y, H, P, N, G, L, num_slots, record_floats, status);
   return launch_status();
 }

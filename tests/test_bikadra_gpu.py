@@ -471,6 +471,47 @@ def test_latent_query_rotation_in_bfloat16(H, dn, rot, dims, pairing):
     assert bool(((outs[0][1].float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
 
 
+@pytest.mark.parametrize("H,P,N,G", [(8, 64, 128, 2), (3, 6, 16, 1), (2, 8, 48, 1), (2, 5, 24, 1)])
+def test_state_space_walk_of_short_portions(H, P, N, G):
+    """Steps whose longest portion is one to five tokens (the walk asks for the inputs of one, two or four tokens together)
+    against the same tokens one by one, bit for bit, and against float64."""
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(H + P)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    rand = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    a_log, dt_bias, d_skip, s0 = rand(H), rand(H), rand(H), rand(7, H, N, P)
+    consts, status = [t.cuda() for t in (dt_bias, a_log, d_skip)], i32([0])
+    for longest in (1, 2, 3, 4, 5):
+        lens, slots = [1, longest, min(2, longest), longest], [5, 0, 3, 6]
+        starts, T = [sum(lens[:i]) for i in range(5)], sum(lens)
+        xbc, proj = rand(T, H * P + 2 * G * N).to(torch.bfloat16), rand(T, 8 + H).to(torch.bfloat16)
+        states, ys = [], []
+        for together in (True, False):
+            state, y = s0.cuda(), torch.full((T, H * P), float("nan"), device="cuda")
+            if together:
+                ops.ssd_scan(xbc.cuda(), proj.cuda(), 8, *consts, state, i32(starts), i32(slots), 4, y, H, P, N, G, status,
+                             max_q_len=longest)
+            else:
+                for b, n in enumerate(lens):
+                    for t in range(starts[b], starts[b] + n):
+                        ops.ssd_scan(xbc[t:t + 1].cuda(), proj[t:t + 1].cuda(), 8, *consts, state, i32([0, 1]), i32([slots[b]]), 1,
+                                     y[t:t + 1], H, P, N, G, status, max_q_len=1)
+            states.append(state)
+            ys.append(y)
+        assert int(status.item()) == 0 and torch.equal(*ys) and torch.equal(*states), longest
+        want, S = torch.empty(T, H, P, dtype=torch.float64), s0.double()
+        for b, n in enumerate(lens):
+            for t in range(starts[b], starts[b] + n):
+                step = torch.nn.functional.softplus(proj[t, 8:].double() + dt_bias.double(), threshold=50)
+                x = xbc[t, :H * P].double().view(H, P)
+                B, C = xbc[t, H * P:].double().view(2, G, N).repeat_interleave(H // G, 1)
+                decay = torch.exp(-a_log.double().exp() * step)
+                S[slots[b]] = decay[:, None, None] * S[slots[b]] + (step[:, None] * B)[:, :, None] * x[:, None]
+                want[t] = torch.einsum("hn,hnp->hp", C, S[slots[b]]) + d_skip.double()[:, None] * x
+        close(ys[0].view(T, H, P), want, "float32")
+        close(states[0], S, "float32")
+
+
 def test_matrix_form_sums_log_decays_in_the_order_of_the_tokens():
     """What a chunk leaves depends on differences of the running sums of its log-decays; summed token by token such a
     difference carries only the roundings of the steps between.  64 heads of 64 x 128, 300 tokens, decays of about one half
