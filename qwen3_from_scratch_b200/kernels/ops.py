@@ -929,6 +929,13 @@ def attn_f32_takes(dtype: torch.dtype, num_q_heads: int, num_kv_heads: int, head
             and num_q_heads // num_kv_heads in (1, 2, 4, 8))
 
 
+def attn_f32_reads(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor, num_seqs: int) -> bool:
+    """Whether the float32 chunk kernels can work on these tensors: they move 16 bytes at a time, and requests and kv heads
+    are dimensions of their grids.  (The plain kernel reads value by value.)"""
+    return (num_seqs <= 65535 and k_pages.shape[1] <= 65535
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_pages, v_pages, out)))
+
+
 ATTN_F32_CHUNK = 64        # keys per chunk: part of the order of a query's additions, not a tuning knob
 ATTN_F32_SCRATCH_CHUNKS = 64
 ATTN_F32_SCRATCH = 1 << 24  # floats
@@ -1235,13 +1242,16 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     Causal attention of a mixed batch over the pages: rows [0, num_decode) bring one token each and
     go to the split-KV decode kernel, the rest to a portion kernel (tcgen05 where it takes the shape,
     else mma.sync; ``portion_kernel="mma"`` forces the latter).  float32 goes to the chunk kernels of csrc/attn_f32.cu
-    (head sizes 64 and 128, up to 8 query heads per kv head); shapes that none of these takes go to the plain kernel."""
+    (head sizes 64 and 128, 1, 2, 4 or 8 query heads per kv head, tensors on 16-byte boundaries); what none of these takes
+    goes to the plain kernel."""
     T, Hq, D = q.shape
     Hkv = k_pages.shape[1]
     if block_table.dim() != 2 or max_kv_len > block_table.shape[1] * k_pages.shape[2]:
         raise KernelError(f"paged_attention: the longest request has {max_kv_len} tokens, a block table row of "
                           f"{block_table.shape[-1]} pages of {k_pages.shape[2]} holds fewer")
-    if attn_f32_takes(q.dtype, Hq, Hkv, D):
+    if attn_f32_takes(q.dtype, Hq, Hkv, D) and attn_f32_reads(q, k_pages, v_pages, out, num_seqs):
+        if partial is not None and (partial.dtype != torch.float32 or not partial.is_contiguous() or partial.data_ptr() % 16):
+            partial = None
         if num_decode > 0:
             attn_f32(q, k_pages, v_pages, out, q_start, kv_len, block_table, num_decode, 1, max_kv_len, scale, window,
                      status, partial)

@@ -289,6 +289,45 @@ def test_attn_f32(hq, hkv, d, page_size, window):
     assert torch.equal(run(single, max(lens)), last)      # no scratch: walked
 
 
+@pytest.mark.parametrize("shifted", ["q", "k", "v", "out", "partial", "none"])
+def test_float32_attention_takes_any_alignment(shifted):
+    """Tensors that do not begin on a 16-byte boundary (which the chunk kernels need) go to the plain kernel, scratch that
+    does not is left alone: single tokens beside a portion against float64."""
+    o = ops()
+    hq, hkv, d, page_size = 4, 2, 64, 16
+    q_lens, kv_lens = [1, 1, 40], [100, 7, 70]
+    q, k_list, v_list, tables, num_pages = attention_case("float32", hq, hkv, d, page_size, kv_lens, q_lens, None, seed=33)
+
+    def place(t, name):
+        """The tensor on the device, one value past a boundary if it is the one under test."""
+        flat = torch.empty(t.numel() + 1, device="cuda")[1 if name == shifted else 0:][:t.numel()]
+        return flat.copy_(t.reshape(-1)).view(t.shape)
+
+    Q, out = place(q, "q"), place(torch.full_like(q, float("nan")), "out")
+    kp, vp = (place(paged(x, page_size, tables, num_pages, torch.float32), n) for x, n in ((k_list, "k"), (v_list, "v")))
+    partial = place(torch.zeros(o.attn_f32_partial_numel(3, hq, d)), "partial")
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))  # noqa: E731
+    st = status()
+    o.paged_attention(Q, kp, vp, out, i32([0, 1, 2, 42]), i32(kv_lens), i32([0, 1] + [2] * 40), dev(table_tensor(tables)), 3, 2, 40,
+                      max(kv_lens), d ** -0.5, 0, st, partial)
+    assert int(st.item()) == 0
+    close(out, reference_attention(q.double(), [k.double() for k in k_list], [v.double() for v in v_list], q_lens, None), "float32")
+
+
+def test_float32_attention_of_more_requests_than_a_grid_dimension_holds():
+    o = ops()
+    n, d = 65537, 64
+    g = torch.Generator().manual_seed(34)
+    q, k, v = torch.randn(n, 1, d, generator=g), torch.randn(1, 1, 4, d, generator=g), torch.randn(1, 1, 4, d, generator=g)
+    every = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    out, st = torch.full((n, 1, d), float("nan"), device="cuda"), status()
+    o.paged_attention(dev(q), dev(k), dev(v), out, every, torch.full((n,), 3, dtype=torch.int32, device="cuda"), every[:n].contiguous(),
+                      torch.zeros(n, 1, dtype=torch.int32, device="cuda"), n, n, 1, 3, d ** -0.5, 0, st)
+    assert int(st.item()) == 0
+    weights = (q[:, 0].double() @ k[0, 0, :3].double().t() * d ** -0.5).softmax(-1)
+    close(out[:, 0], weights @ v[0, 0, :3].double(), "float32")
+
+
 def test_attn_f32_reports_bad_tables():
     """A page outside the pool and a context beyond what the launch was made for are reported, not read; a value that a
     query does not see takes no part in its sum, even if it is not a number."""
