@@ -4,7 +4,8 @@
 // A query's result depends only on its own keys, not on how the batch was cut or on the kernel that computes it.  The keys
 // are taken in chunks of 64 by their absolute position, and for each chunk that holds a key the query sees:
 //   s_n = scale * (q . k_n)        the dot product by runs of 16 values, the runs added one after the other
-//   m_c = max s_n,  p_n = exp(s_n - m_c),  l_c = sum p_n (keys t, t + 16, t + 32, t + 48 first, then over t by halves)
+//   m_c = max s_n                  no lower than the lowest finite number
+//   p_n = exp(s_n - m_c),  l_c = sum p_n  (keys t, t + 16, t + 32, t + 48 first, then over t by halves)
 //   o_c = sum p_n v_n              ascending n
 // and the chunks are folded together in ascending order: m' = max(m, m_c), l' = l exp(m - m') + l_c exp(m_c - m'), o likewise.
 // Long contexts keep their accuracy (sums of 64, then one term per chunk), and the chunks of a single token can be
@@ -17,12 +18,17 @@
 // a warp per token and head) took 1,435, 6,600 and 453 us: some 1.6 us per key of the longest context, whatever the batch.
 //
 // Reference formulas: as in attn_ref.cu (models/attn.py:402-499, kernels/triton/paged_attn.py:89-181).
+#include <float.h>
+
 #include "common.cuh"
 
 namespace q3 {
 
 constexpr int AF_THREADS = 128, AF_CHUNK = 64;
 constexpr float AF_MASKED = -1.0f;  // in place of a probability: the query does not see the key
+// The maximum of a chunk is at least this if the query sees a key of it: where all the scores that it sees have fallen to
+// minus infinity their weights are 0, not exp(-inf + inf), and the chunks beside it keep their values.
+constexpr float AF_LOWEST = -FLT_MAX;
 
 __device__ __forceinline__ void af_copy16(uint32_t dst, const float* src, bool in) {
   const int n = in ? 16 : 0;  // zero bytes read: the destination is filled with zeros
@@ -41,7 +47,7 @@ struct AfShape {
 // Bound by shared-memory reads and the FMA pipe together (a 4 x 4 piece of the scores per thread: 8 reads of 16 bytes for
 // 64 FMA); K of the next chunk is fetched under P V, V under the scores.
 template <int D, int RPT>
-__global__ void __launch_bounds__(AF_THREADS)
+__global__ void __launch_bounds__(AF_THREADS, D == 128 ? 2 : 3)  // (what an SM's shared memory holds)
 attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                 float* __restrict__ out, const int* __restrict__ q_start, const int* __restrict__ kv_len,
                 const int* __restrict__ block_table, int table_stride, int page_size, int num_pages, int Hq, int Hkv,
@@ -160,11 +166,14 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         bool sees[4];
-        mc[i] = -INFINITY;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int key = tx + 16 * j, n = chunk * AF_CHUNK + key;
           sees[j] = n >= lo[i] && n <= pos[i] && ((ok >> key) & 1ull);
+        }
+        mc[i] = sees[0] || sees[1] || sees[2] || sees[3] ? AF_LOWEST : -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
           s[i][j] = __fmul_rn(s[i][j], scale);  // (not contracted with the subtraction below)
           if (sees[j]) mc[i] = fmaxf(mc[i], s[i][j]);
         }
@@ -232,7 +241,7 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
   for (int i = 0; i < RPT; ++i) {
     const int r = ty + 8 * i;
     if (r >= live_rows) continue;
-    const float inv = l[i] == 0.f ? 0.f : 1.0f / l[i];
+    const float inv = l[i] == 0.f && m[i] == -INFINITY ? 0.f : 1.0f / l[i];  // 0: no key seen
     float* dst = out + ((size_t)(t0 + tok0 + r / G) * Hq + hk * G + r % G) * D;
 #pragma unroll
     for (int c = 0; c < DV; ++c)
@@ -247,7 +256,7 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
 // column for P V (4 requests at contexts of 400 to 900, 16 heads over 8 of 128: 14.5 us with the kernel above cut by chunks,
 // one of whose warps had rows, 13.0 us here; batch 1 at 4,096: 69 and 36 us with the fold).
 template <int D, int G>
-__global__ void __launch_bounds__(AF_THREADS)
+__global__ void __launch_bounds__(AF_THREADS, D == 128 ? 3 : 6)
 attn_f32_chunk_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                       float* __restrict__ partial, const int* __restrict__ q_start, const int* __restrict__ kv_len,
                       const int* __restrict__ block_table, int table_stride, int page_size, int num_pages, int Hq, int Hkv,
@@ -340,7 +349,7 @@ attn_f32_chunk_kernel(const float* __restrict__ q, const float* __restrict__ k_p
       const int key = tx + 16 * j, n = chunk * AF_CHUNK + key;
       s[j] = head < G ? p_s[head][key] : 0.f;
       sees[j] = n >= lo && n <= pos && ((ok >> key) & 1ull);
-      if (sees[j]) mc = fmaxf(mc, s[j]);
+      if (sees[j]) mc = fmaxf(mc, fmaxf(s[j], AF_LOWEST));
     }
 #pragma unroll
     for (int x = 8; x > 0; x >>= 1) mc = fmaxf(mc, __shfl_xor_sync(0xffffffffu, mc, x));
@@ -415,7 +424,7 @@ attn_f32_fold_kernel(const float* __restrict__ partial, float* __restrict__ out,
       }
     }
   }
-  out[((size_t)t * Hq + head) * D + d] = l == 0.f ? 0.f : o * (1.0f / l);
+  out[((size_t)t * Hq + head) * D + d] = l == 0.f && m == -INFINITY ? 0.f : o * (1.0f / l);
 }
 
 template <int D, int G>

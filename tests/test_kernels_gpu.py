@@ -328,6 +328,42 @@ def test_float32_attention_of_more_requests_than_a_grid_dimension_holds():
     close(out[:, 0], weights @ v[0, 0, :3].double(), "float32")
 
 
+@pytest.mark.parametrize("single", [True, False])
+def test_attn_f32_with_scores_of_minus_infinity(single):
+    """Scores that have fallen to minus infinity weigh nothing, a whole chunk of them included, as in the plain kernel; a
+    query that sees nothing else has no result (not a number), one that sees a score that is not a number neither."""
+    o = ops()
+    hq, hkv, d, page_size, n = 4, 2, 64, 16, 200
+    q, k_list, v_list, tables, num_pages = attention_case("float32", hq, hkv, d, page_size, [n], [n], None, seed=35)
+    q = q.abs() + 0.1
+
+    def run(k, rows, f32):
+        kp, vp = (dev(paged([x], page_size, tables, num_pages, torch.float32)) for x in (k, v_list[0]))
+        Q, table, st = dev(q)[n - rows:].contiguous(), dev(table_tensor(tables)), status()
+        out, q_start = torch.full_like(Q, 7.0), dev(torch.tensor([0, rows], dtype=torch.int32))
+        kv_len, tok_seq = dev(torch.tensor([n], dtype=torch.int32)), torch.zeros(rows, dtype=torch.int32, device="cuda")
+        if f32:
+            partial = torch.empty(o.attn_f32_partial_numel(1, hq, d), device="cuda") if single else None
+            o.attn_f32(Q, kp, vp, out, q_start, kv_len, table, 1, rows, n, d ** -0.5, 0, st, partial)
+        else:
+            o.attn_ref(Q, kp, vp, out, q_start, kv_len, tok_seq, table, d ** -0.5, 0, st)
+        assert int(st.item()) == 0
+        return out
+
+    rows = 1 if single else 60
+    for low in ((64, 128), (70, 90), (1, 200)):  # a whole chunk, part of one, all but the first key
+        k = k_list[0].clone()
+        k[low[0]:low[1]] = -3e38  # the products' sum overflows
+        got = run(k, rows, True)
+        assert bool(torch.isfinite(got).all())
+        close(got, run(k, rows, False), "float32")
+    k = torch.full_like(k_list[0], -3e38)
+    assert bool(torch.isnan(run(k, rows, True)).all()) and bool(torch.isnan(run(k, rows, False)).all())
+    k = k_list[0].clone()
+    k[64:128] = float("nan")
+    assert bool(torch.isnan(run(k, rows, True)).all())
+
+
 def test_attn_f32_reports_bad_tables():
     """A page outside the pool and a context beyond what the launch was made for are reported, not read; a value that a
     query does not see takes no part in its sum, even if it is not a number."""
