@@ -3,7 +3,9 @@
 //
 // A query's result depends only on its own keys, not on how the batch was cut or on the kernel that computes it.  The keys
 // are taken in chunks of 64 by their absolute position, and for each chunk that holds a key the query sees:
-//   s_n = scale * (q . k_n)        the dot product by runs of 16 values, the runs added one after the other
+//   s_n = scale * (q . k_n)        the dot product by runs of 32 values: eight chains of 4, added by halves, and the runs one
+//                                  after the other (as close to 64 bits as the shuffle tree of attn_ref.cu; with chains of
+//                                  16 the results for 2 to 65 keys were 2 to 11 % further off than that kernel's)
 //   m_c = max s_n                  no lower than the lowest finite number
 //   p_n = exp(s_n - m_c),  l_c = sum p_n  (keys t, t + 16, t + 32, t + 48 first, then over t by halves)
 //   o_c = sum p_n v_n              ascending n
@@ -35,6 +37,9 @@ __device__ __forceinline__ void af_copy16(uint32_t dst, const float* src, bool i
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ float4 af_lds(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float af_dot4(float4 a, float4 b) {  // a chain; __fmul_rn: never joined with an addition of its result
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, __fmul_rn(a.x, b.x))));
+}
 
 // RPT: rows per thread; the block has 8 RPT (token, head) rows of one kv head, row r = token r / G, head r % G of the group.
 template <int D, int RPT>
@@ -139,29 +144,39 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
 #pragma unroll 1
-      for (int run = 0; run < D / 16; ++run) {
-        float part[RPT][4];
+      for (int run = 0; run < D / 32; ++run) {
+        float whole[RPT][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float4 kv[4];
+        for (int half = 0; half < 2; ++half) {
+          float two[RPT][4], other[RPT][4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) kv[j] = af_lds(k_s + (tx + 16 * j) * D + (((run * 4 + c) ^ (tx & 7)) * 4));
+          for (int c = 0; c < 4; ++c) {
+            const int piece = run * 8 + half * 4 + c;
+            float4 kv[4];
 #pragma unroll
-          for (int i = 0; i < RPT; ++i) {
-            const float4 a = af_lds(q_s + (ty + 8 * i) * D + (((run * 4 + c) ^ ty) * 4));
+            for (int j = 0; j < 4; ++j) kv[j] = af_lds(k_s + (tx + 16 * j) * D + ((piece ^ (tx & 7)) * 4));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              part[i][j] = c == 0 ? a.x * kv[j].x : fmaf(a.x, kv[j].x, part[i][j]);
-              part[i][j] = fmaf(a.y, kv[j].y, part[i][j]);
-              part[i][j] = fmaf(a.z, kv[j].z, part[i][j]);
-              part[i][j] = fmaf(a.w, kv[j].w, part[i][j]);
+            for (int i = 0; i < RPT; ++i) {
+              const float4 a = af_lds(q_s + (ty + 8 * i) * D + ((piece ^ ty) * 4));
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float p = af_dot4(a, kv[j]);
+                if (c == 0) two[i][j] = p;
+                else if (c == 1) two[i][j] += p;
+                else if (c == 2) other[i][j] = p;
+                else other[i][j] += p;
+              }
             }
           }
+#pragma unroll
+          for (int i = 0; i < RPT; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float sum16 = two[i][j] + other[i][j];
+              if (half == 0) whole[i][j] = sum16;
+              else s[i][j] += whole[i][j] + sum16;
+            }
         }
-#pragma unroll
-        for (int i = 0; i < RPT; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) s[i][j] += part[i][j];
       }
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
@@ -316,22 +331,31 @@ attn_f32_chunk_kernel(const float* __restrict__ q, const float* __restrict__ k_p
 #pragma unroll
     for (int i = 0; i < RH; ++i) s[i] = 0.f;
 #pragma unroll 2
-    for (int run = 0; run < D / 16; ++run) {
-      float part[RH];
+    for (int run = 0; run < D / 32; ++run) {
+      float whole[RH];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float4 kv = af_lds(k_s + key * D + (((run * 4 + c) ^ (key & 7)) * 4));
+      for (int half = 0; half < 2; ++half) {
+        float two[RH], other[RH];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int piece = run * 8 + half * 4 + c;
+          const float4 kv = af_lds(k_s + key * D + ((piece ^ (key & 7)) * 4));
+#pragma unroll
+          for (int i = 0; i < RH; ++i) {
+            const float p = af_dot4(af_lds(&q_s[min((tid >> 6) + 2 * i, G - 1)][piece * 4]), kv);
+            if (c == 0) two[i] = p;
+            else if (c == 1) two[i] += p;
+            else if (c == 2) other[i] = p;
+            else other[i] += p;
+          }
+        }
 #pragma unroll
         for (int i = 0; i < RH; ++i) {
-          const float4 a = af_lds(&q_s[min((tid >> 6) + 2 * i, G - 1)][(run * 4 + c) * 4]);
-          part[i] = c == 0 ? a.x * kv.x : fmaf(a.x, kv.x, part[i]);
-          part[i] = fmaf(a.y, kv.y, part[i]);
-          part[i] = fmaf(a.z, kv.z, part[i]);
-          part[i] = fmaf(a.w, kv.w, part[i]);
+          const float sum16 = two[i] + other[i];
+          if (half == 0) whole[i] = sum16;
+          else s[i] += whole[i] + sum16;
         }
       }
-#pragma unroll
-      for (int i = 0; i < RH; ++i) s[i] += part[i];
     }
 #pragma unroll
     for (int i = 0; i < RH; ++i)
