@@ -923,10 +923,16 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages: 
     _done("gemm_tc_qkv", code, f"T {T} K {K} heads {num_q_heads}/{num_kv_heads} x {head_dim}{' pair' if pair else ''}")
 
 
-def attn_f32_takes(dtype: torch.dtype, num_q_heads: int, num_kv_heads: int, head_dim: int) -> bool:
-    """Whether the float32 chunk kernels take this shape (else the plain kernel runs)."""
+ATTN_F32_PLAIN_WINDOW = 16
+
+
+def attn_f32_takes(dtype: torch.dtype, num_q_heads: int, num_kv_heads: int, head_dim: int, window: int = 0) -> bool:
+    """Whether the float32 chunk kernels take this shape (else the plain kernel runs).  The shortest windows stay with the
+    plain kernel, which walks over their few keys while a chunk kernel brings 64 or 128 (300 tokens on 16 heads over 8 of 128:
+    a window of 8 12.6 us against 26, of 16 22 and 27, of 24 32 and 28; 64 single tokens: 16 14.6 and 14.5).  The window is the
+    layer's, so a token's bits do not depend on its step."""
     return (dtype == torch.float32 and head_dim in (64, 128) and num_q_heads % num_kv_heads == 0
-            and num_q_heads // num_kv_heads in (1, 2, 4, 8))
+            and num_q_heads // num_kv_heads in (1, 2, 4, 8) and not 0 < window <= ATTN_F32_PLAIN_WINDOW)
 
 
 def attn_f32_reads(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor, num_seqs: int) -> bool:
@@ -1242,14 +1248,14 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     Causal attention of a mixed batch over the pages: rows [0, num_decode) bring one token each and
     go to the split-KV decode kernel, the rest to a portion kernel (tcgen05 where it takes the shape,
     else mma.sync; ``portion_kernel="mma"`` forces the latter).  float32 goes to the chunk kernels of csrc/attn_f32.cu
-    (head sizes 64 and 128, 1, 2, 4 or 8 query heads per kv head, tensors on 16-byte boundaries); what none of these takes
-    goes to the plain kernel."""
+    (head sizes 64 and 128, 1, 2, 4 or 8 query heads per kv head, windows beyond 16, tensors on 16-byte boundaries); what none
+    of these takes goes to the plain kernel."""
     T, Hq, D = q.shape
     Hkv = k_pages.shape[1]
     if block_table.dim() != 2 or max_kv_len > block_table.shape[1] * k_pages.shape[2]:
         raise KernelError(f"paged_attention: the longest request has {max_kv_len} tokens, a block table row of "
                           f"{block_table.shape[-1]} pages of {k_pages.shape[2]} holds fewer")
-    if attn_f32_takes(q.dtype, Hq, Hkv, D) and attn_f32_reads(q, k_pages, v_pages, out, num_seqs):
+    if attn_f32_takes(q.dtype, Hq, Hkv, D, window) and attn_f32_reads(q, k_pages, v_pages, out, num_seqs):
         if partial is not None and (partial.dtype != torch.float32 or not partial.is_contiguous() or partial.data_ptr() % 16):
             partial = None
         if num_decode > 0:

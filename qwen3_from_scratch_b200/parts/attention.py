@@ -84,7 +84,7 @@ class GQAAttention(Mixer):
         if ops.fast_attention_takes(rt.dtype, self.num_heads, self.num_kv_heads, self.head_dim):
             self._partial = rt.shared("attn.partial", ops.decode_partial_numel(rt.max_seqs, self.num_heads,
                                                                                self.head_dim), dtype=torch.float32)
-        elif ops.attn_f32_takes(rt.dtype, self.num_heads, self.num_kv_heads, self.head_dim):
+        elif ops.attn_f32_takes(rt.dtype, self.num_heads, self.num_kv_heads, self.head_dim, self.window or 0):
             self._partial = rt.shared("attn.partial", ops.attn_f32_partial_numel(rt.max_seqs, self.num_heads,
                                                                                  self.head_dim), dtype=torch.float32)
 

@@ -387,6 +387,30 @@ def test_attn_f32_is_no_further_from_64_bits_than_the_plain_kernel(hq, hkv, d, n
     assert errors[0] <= 1.03 * errors[1], errors
 
 
+@pytest.mark.parametrize("window", [1, 16, 17, 63, 64, 65, 66, 127, 128, 129, 130, 1000, 2 ** 31 - 1])
+def test_float32_attention_in_windows(window):
+    """Single tokens in a window (blocks only for the chunks that it reaches, the shortest windows on the plain kernel) give
+    the bits that the same tokens get as a portion's, and agree with float64."""
+    o = ops()
+    hq, hkv, d, page_size = 4, 2, 64, 16
+    lens = [1, 2, 16, 63, 64, 65, 80, 127, 128, 129, 191, 192, 193, 300]
+    q, k_list, v_list, tables, num_pages = attention_case("float32", hq, hkv, d, page_size, lens, lens, None, seed=37)
+    kp, vp = (dev(paged(x, page_size, tables, num_pages, torch.float32)) for x in (k_list, v_list))
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))  # noqa: E731
+    table = torch.nn.functional.pad(table_tensor(tables), (0, 64 - table_tensor(tables).shape[1]), value=-1).cuda()
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    whole, st, B = torch.full_like(dev(q), float("nan")), status(), len(lens)
+    o.paged_attention(dev(q), kp, vp, whole, i32(starts), i32(lens), i32([b for b, n in enumerate(lens) for _ in range(n)]), table, B, 1,
+                      max(lens), max(lens), d ** -0.5, window, st)
+    close(whole, reference_attention(q.double(), [k.double() for k in k_list], [v.double() for v in v_list], lens,
+                                     window if window < 1000 else None), "float32")
+    last = [s - 1 for s in starts[1:]]
+    out, partial = torch.full((B, hq, d), float("nan"), device="cuda"), torch.full((o.attn_f32_partial_numel(B, hq, d),), float("nan"), device="cuda")
+    o.paged_attention(dev(q[last]), kp, vp, out, i32(list(range(B + 1))), i32(lens), i32(list(range(B))), table, B, B, 1, 1024, d ** -0.5,
+                      window, st, partial)  # the context bucket of a recorded step
+    assert int(st.item()) == 0 and torch.equal(out, whole[last])
+
+
 def test_attn_f32_reports_bad_tables():
     """A page outside the pool and a context beyond what the launch was made for are reported, not read; a value that a
     query does not see takes no part in its sum, even if it is not a number."""
