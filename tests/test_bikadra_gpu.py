@@ -12,7 +12,7 @@ import pytest
 import torch
 
 import plain_bikadra as plain
-from bikadra_models import CONFIGS, make_folder
+from bikadra_models import CONFIGS, latent, make_folder, mamba2
 from harness import Replayer, assert_close
 from test_binupel_gpu import MixerBench, part_weights
 
@@ -131,6 +131,28 @@ def test_dense_feed_forward_in_every_product(rows, dtype):
     x = torch.randn(rows, 64, generator=torch.Generator().manual_seed(rows + 1)).to(DT[dtype])
     want = plain.dense_ff(x.double(), ref, "")
     close(part.forward(x.cuda()), want, dtype, f"dense feed-forward, {rows} rows")
+
+
+@pytest.mark.parametrize("rows,width", [(1023, 64), (1024, 64), (1100, 72), (511, 1544), (512, 1544)])
+@pytest.mark.parametrize("activation", ["silu", "relu", "gelu_tanh", "relu_sq"])
+def test_dense_feed_forward_of_many_rows(rows, width, activation, monkeypatch):
+    """The part on both sides of the line from which the activation runs in the paired tcgen05 product's epilogue (1,024
+    rows, 512 where the reduction is long), against float64."""
+    from qwen3_from_scratch_b200.kernels import ops
+    from qwen3_from_scratch_b200.parts.base import PartSpec, Runtime
+    from qwen3_from_scratch_b200.registry import create_part
+    part = create_part("feed_forward", PartSpec("dense_mlp", {"hidden_size": width, "intermediate_size": 200, "activation": activation,
+                                                              "names": {"up": "up", "down": "down"}}), name="f")
+    dev, ref = part_weights(part, "bfloat16", seed=rows)
+    rt = Runtime(torch.device("cuda:0"), torch.bfloat16, 1100, 2)
+    part.setup(rt, dict(dev))
+    fused, act = [], ops.gemm_tc_act
+    monkeypatch.setattr(ops, "gemm_tc_act", lambda *args: (fused.append(1), act(*args)))
+    x = torch.randn(rows, width, generator=torch.Generator().manual_seed(rows + 1)).to(torch.bfloat16)
+    f, z = torch.nn.functional, x.double() @ ref["up"].t()
+    h = {"silu": f.silu(z), "relu": z.relu(), "gelu_tanh": f.gelu(z, approximate="tanh"), "relu_sq": z.relu() ** 2}[activation]
+    close(part.forward(x.cuda()), h @ ref["down"].t(), "bfloat16", f"{rows} rows of {width}, {activation}")
+    assert len(fused) == (1 if rows in (1024, 1100, 512) else 0) and int(rt.status.item()) == 0
 
 
 # ---------------------------------------------------------------------- each mixer alone
@@ -726,6 +748,69 @@ def test_long_prompt_on_the_serving_kernels(folders):
         got = replay(folders["z"], "bfloat16", {"a": ids}, lambda r, cuts=cuts: [r.step([("a", n)]) for n in cuts],
                      page_size=16, num_pages=64, max_seqs=2, max_step_tokens=1024)
         assert_close(got, want, "bfloat16", f"z long {name}", tol=tol)
+
+
+# heads of 128 + 64 and 128, the sizes whose portions attend over formed keys and values; two latent ranks, a loop
+FORMED = {
+    "architecture": "Bikadra", "vocab": 211, "width": 64, "embedding": {"scale": 4.0}, "streams": 2, "norm": {"eps": 1e-5},
+    "loop": {"start": 0, "stop": 2, "times": 2},
+    "layers": [latent(3, 128, 64, 128, 64, 48, 0.07, 10000.0, scaling=(4.0, 64, 8.0, 1.0), ff=72),
+               mamba2(6, 16, 24, 3, 2, 4, ff=80),
+               latent(2, 128, 64, 128, 128, 40, 0.1, 500.0, dims=32, ff=None)]}
+
+
+def test_model_whose_portions_attend_over_formed_keys(tmp_path, monkeypatch):
+    """The attention part's choice between formed and absorbed latents through whole models: prompts whole, in portions on
+    both sides of the rule (which needs 32 tokens for each 1,024 rows), beside single tokens, by more requests than the rows
+    hold, and steps of one shape often enough to be recorded and replayed.  Which form ran is counted."""
+    from qwen3_from_scratch_b200.engine.session import Session
+    from qwen3_from_scratch_b200.kernels import ops
+    folder = make_folder(str(tmp_path / "formed"), FORMED, 6)
+    cfg, w = plain.read_model_folder(folder)
+    calls = []
+    for name in ("latent_attention_formed", "latent_attention"):
+        def counted(*args, _fn=getattr(ops, name), _name=name, **kwargs):
+            calls.append(_name)
+            return _fn(*args, **kwargs)
+        monkeypatch.setattr(ops, name, counted)
+
+    def took(form, fn):
+        calls.clear()
+        fn()
+        assert set(calls) == {form}, (form, calls)
+
+    formed, absorbed = "latent_attention_formed", "latent_attention"
+    lens = {"a": 400, "b": 330, "c": 40, "d": 33, "e": 35, "f": 300}
+    seqs = {r: tokens(cfg["vocab"], n, 100 + i) for i, (r, n) in enumerate(lens.items())}
+    want = {r: plain.forward_logits(cfg, w, ids) for r, ids in seqs.items()}
+    tol = tolerance("bfloat16", cfg, w, seqs)
+    session = Session(folder, dtype="bfloat16", page_size=16, num_pages=96, max_seqs=6, max_step_tokens=512)
+    r = Replayer(session, seqs)
+    took(formed, lambda: r.step([("a", 300)]))                               # tiles of 128 rows and keys, and a ragged one
+    took(formed, lambda: r.step([("b", 32)]))
+    took(absorbed, lambda: r.step([("b", 31)]))
+    took(absorbed, lambda: r.step([("a", 1)]))
+    took(absorbed, lambda: r.step([("a", 40), ("b", 1)]))                    # a single token in the step
+    took(formed, lambda: r.step([("a", 59), ("b", 129)]))                    # a ends
+    r.step([("b", 1)])                                                       # the single token's step again: replayed
+    took(formed, lambda: r.step([("c", 38), ("d", 33), ("e", 33), ("b", 30)]))  # four requests: all the rows there are; d ends
+    took(absorbed, lambda: r.step([("c", 2), ("e", 2), ("f", 100), ("b", 2)]))  # too few tokens for so many rows; c and e end
+    replays = session.step_graphs.replays
+    for i in range(5):
+        calls.clear()
+        r.step([("f", 40)])  # runs, runs and is recorded, is replayed
+        assert set(calls) == ({formed} if i < 2 else set()), (i, calls)
+    assert session.step_graphs.replays == replays + 3
+    while r.remaining("b"):
+        r.step([("b", 1)])
+    session.manager.check()
+    assert session.manager.free_slots() == 6
+    assert_close(r.result(), want, "bfloat16", "formed and absorbed", tol=tol)
+    many = {i: tokens(cfg["vocab"], 50, 120 + i) for i in range(5)}  # five requests: more rows than there are
+    r = Replayer(session, many)
+    took(absorbed, lambda: r.step([(i, 50) for i in many]))
+    assert_close(r.result(), {i: plain.forward_logits(cfg, w, ids) for i, ids in many.items()}, "bfloat16", "five requests",
+                 tol=tolerance("bfloat16", cfg, w, many))
 
 
 def test_long_decoding_through_graphs(folders):
