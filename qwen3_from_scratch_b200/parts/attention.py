@@ -315,10 +315,12 @@ class LatentAttention(Mixer):
         # the attended latent out; both in the compute dtype (a float32 run: float32)
         self.uk_t = uk.view(H, self.dim, self.kv_rank).transpose(1, 2).to(rt.dtype).contiguous()
         self.uv = uv.view(H, self.vdim, self.kv_rank).to(rt.dtype).contiguous()
-        # prompt portions form the heads' keys and values instead: both weights as one product over the latents
+        # prompt portions form the heads' keys and values instead: both weights as one product over the latents, of which
+        # W_uv is the second half as it stands
         self.formed = ops.latent_formed_takes(rt.dtype, self.dim, self.rot_dim, self.vdim, self.kv_rank, self.scale)
         if self.formed:
-            self.kv_up_t = torch.cat([uk.to(rt.dtype), uv.to(rt.dtype)], dim=0).t()
+            kv_up = torch.cat([uk.to(rt.dtype), uv.to(rt.dtype)], dim=0)
+            self.kv_up_t, self.uv = kv_up.t(), kv_up[H * self.dim:].view(H, self.vdim, self.kv_rank)
             rows = ops.latent_formed_rows(rt.max_tokens)
             self._c_rows = rt.shared("lattn.c_rows", rows, self.kv_rank)
             self._r_rows = rt.shared("lattn.r_rows", rows, self.rot_dim)

@@ -813,6 +813,17 @@ def test_model_whose_portions_attend_over_formed_keys(tmp_path, monkeypatch):
                  tol=tolerance("bfloat16", cfg, w, many))
 
 
+def test_latent_attention_keeps_the_value_weights_once(tmp_path):
+    """The weights that form keys and values hold W_uv as the absorbed form reads it: not a second copy."""
+    from qwen3_from_scratch_b200.engine.session import Session
+    folder = make_folder(str(tmp_path / "formed"), FORMED, 6)
+    session = Session(folder, dtype="bfloat16", page_size=16, num_pages=8, max_seqs=2, max_step_tokens=64)
+    found = [block.mixer for block in session.model.layers if getattr(block.mixer, "formed", False)]
+    assert len(found) == 2
+    for m in found:
+        assert m.uv.untyped_storage().data_ptr() == m.kv_up_t.untyped_storage().data_ptr()
+
+
 def test_long_decoding_through_graphs(folders):
     """300 single tokens after a short prompt, replayed from CUDA graphs: states and latents are carried on the
     device from step to step; the last logits still agree with the plain implementation in float32."""
