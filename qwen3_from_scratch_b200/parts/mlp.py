@@ -155,7 +155,7 @@ class DenseMLP(FeedForward):
             return self.down(h)
         if (self.rt.dtype == torch.bfloat16 and not self.up.full_precision and x.dtype == torch.bfloat16
                 and self.activation in ops.GEMM_TC_ACTIVATIONS and ops.gemm_tc_act_pays(rows, self.up.weight)
-                and ops.gemm_tc_takes(x, self.up.weight)):
+                and ops.gemm_tc_takes(x, self.up.weight) and x.is_contiguous() and x.data_ptr() % 16 == 0):
             # prompt portions: the activation in the product's epilogue
             h = self.up._buffer("_out", rows, self.up.out_dtype)
             ops.gemm_tc_act(x, self.up.weight, h, self.activation, self.rt.status)

@@ -155,6 +155,24 @@ def test_dense_feed_forward_of_many_rows(rows, width, activation, monkeypatch):
     assert len(fused) == (1 if rows in (1024, 1100, 512) else 0) and int(rt.status.item()) == 0
 
 
+@pytest.mark.parametrize("layout", ["columns of a wider tensor", "off a 16-byte boundary"])
+def test_dense_feed_forward_of_many_rows_takes_any_layout(layout):
+    """Inputs that the tcgen05 product does not read go through the library's product, as they did before there was one."""
+    from qwen3_from_scratch_b200.parts.base import PartSpec, Runtime
+    from qwen3_from_scratch_b200.registry import create_part
+    part = create_part("feed_forward", PartSpec("dense_mlp", {"hidden_size": 64, "intermediate_size": 136,
+                                                              "activation": "gelu_tanh", "names": {"up": "up", "down": "down"}}),
+                       name="f")
+    dev, ref = part_weights(part, "bfloat16", seed=3)
+    part.setup(Runtime(torch.device("cuda:0"), torch.bfloat16, 1100, 2), dict(dev))
+    x = torch.randn(1100, 64, generator=torch.Generator().manual_seed(4)).to(torch.bfloat16)
+    if layout == "off a 16-byte boundary":
+        given = torch.empty(1100 * 64 + 1, dtype=torch.bfloat16, device="cuda")[1:].view(1100, 64)
+    else:
+        given = torch.empty(1100, 72, dtype=torch.bfloat16, device="cuda")[:, 8:]
+    close(part.forward(given.copy_(x)), plain.dense_ff(x.double(), ref, ""), "bfloat16", layout)
+
+
 # ---------------------------------------------------------------------- each mixer alone
 def _latent(params):
     m = {"heads": params["num_heads"], "dim": params["dim"], "rot_dim": params["rot_dim"], "vdim": params["vdim"],
