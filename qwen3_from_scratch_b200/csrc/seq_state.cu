@@ -342,23 +342,23 @@ block_diag_kernel(const T* __restrict__ u, const T* __restrict__ w, float* __res
 // multiply-adds each, so that both operands come in pieces of 16 bytes and all tokens are under way at once; the lanes'
 // sums meet in the order of warp_sum.  The tokens' values are brought into shared memory once per block, as float32; the
 // weights are asked for before the wait.  Bound by the chain of latencies (load, products, reduction): 8 blocks of 512 x 256,
-// 8 tokens 3.9 us, one 2.0 us; 13.8 and 3.9 us with the kernel above.  Tensor cores would do it in 2.3 us, but their sums are
+// 8 tokens 3.3 us, one 2.0 us; 13.8 and 3.9 us with the kernel above.  Tensor cores would do it in 2.3 us, but their sums are
 // 2.0 to 2.5 times further from 64 bits.
-constexpr int BDR_WARPS = 4, BDR_ROWS = BDR_WARPS * 8;
 constexpr int BDR_MAX_TOKENS = 16;
 
 __device__ __forceinline__ float bf16_of(uint32_t w, int i) {  // value i of a word's two
   return __uint_as_float(i ? w & 0xffff0000u : w << 16);
 }
 
-template <int MT>
-__global__ void __launch_bounds__(BDR_WARPS * 32)
+// Grid (8 WARPS rows of a block of w, blocks of w, groups of MT tokens).
+template <int MT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 block_diag_rows_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ w, float* __restrict__ out,
                        int Ttot, int C, int bw, int rows) {
   constexpr int BATCH = MT <= 4 ? 8 : 4;  // pieces of a row asked for together
   extern __shared__ __align__(16) float bd_tokens[];  // [MT][bw]
   const int lane = threadIdx.x & 31, q = lane & 3;
-  const int blk = blockIdx.y, r = (blockIdx.x * BDR_WARPS + (threadIdx.x >> 5)) * 8 + (lane >> 2);
+  const int blk = blockIdx.y, r = (blockIdx.x * WARPS + (threadIdx.x >> 5)) * 8 + (lane >> 2), t0 = blockIdx.z * MT;
   const __nv_bfloat16* wr = w + ((size_t)blk * rows + min(r, rows - 1)) * bw + 8 * q;
   const int steps = (bw - 8 * q + 31) / 32;  // this thread's pieces: values 32 k + 8 q .. + 7
   uint4 cur[BATCH], next[BATCH];
@@ -370,10 +370,10 @@ block_diag_rows_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16*
   load(cur, 0);
   pdl_wait();
   pdl_launch_dependents();
-  for (int i = threadIdx.x; i < MT * (bw / 8); i += BDR_WARPS * 32) {
+  for (int i = threadIdx.x; i < MT * (bw / 8); i += WARPS * 32) {
     const int t = i / (bw / 8), c = i % (bw / 8);
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (t < Ttot) v = *reinterpret_cast<const uint4*>(u + (size_t)t * C + (size_t)blk * bw + c * 8);
+    if (t0 + t < Ttot) v = *reinterpret_cast<const uint4*>(u + (size_t)(t0 + t) * C + (size_t)blk * bw + c * 8);
     float* dst = bd_tokens + t * bw + c * 8;
     *reinterpret_cast<float4*>(dst) = make_float4(bf16_of(v.x, 0), bf16_of(v.x, 1), bf16_of(v.y, 0), bf16_of(v.y, 1));
     *reinterpret_cast<float4*>(dst + 4) = make_float4(bf16_of(v.z, 0), bf16_of(v.z, 1), bf16_of(v.w, 0), bf16_of(v.w, 1));
@@ -415,18 +415,18 @@ block_diag_rows_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16*
     for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
       for (int e = 0; e < o; ++e) v[e] += v[e + o];
-    if (r < rows && t < Ttot && (t & 3) == q) out[((size_t)blk * Ttot + t) * rows + r] = v[0];
+    if (r < rows && t0 + t < Ttot && (t & 3) == q) out[((size_t)blk * Ttot + t0 + t) * rows + r] = v[0];
   }
 }
 
-template <int MT>
+template <int MT, int WARPS>
 static int block_diag_rows_launch(const void* u, const void* w, float* out, int T, int nb, int bw, int rows, cudaStream_t stream) {
   constexpr int most = MT * 32 * BD_MAX_PER_LANE * (int)sizeof(float);
   if (most > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(block_diag_rows_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const cudaError_t e = cudaFuncSetAttribute(block_diag_rows_kernel<MT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return (int)e;
   }
-  launch(block_diag_rows_kernel<MT>, dim3((rows + BDR_ROWS - 1) / BDR_ROWS, nb), dim3(BDR_WARPS * 32),
+  launch(block_diag_rows_kernel<MT, WARPS>, dim3((rows + 8 * WARPS - 1) / (8 * WARPS), nb, (T + MT - 1) / MT), dim3(WARPS * 32),
          (size_t)MT * bw * sizeof(float), stream, (const __nv_bfloat16*)u, (const __nv_bfloat16*)w, out, T, nb * bw, bw, rows);
   return launch_status();
 }
@@ -918,11 +918,17 @@ extern "C" int q3_block_diag(const void* u, const void* w, float* out, int dtype
   if (bw <= 0) return Q3_ERR_SIZE;
   if (dtype == Q3_BF16 && T <= q3::BDR_MAX_TOKENS && bw % 8 == 0 && bw <= 32 * q3::BD_MAX_PER_LANE && nb <= 65535 &&
       (uintptr_t)u % 16 == 0 && (uintptr_t)w % 16 == 0) {
-    if (T == 1) return q3::block_diag_rows_launch<1>(u, w, out, T, nb, bw, rows, stream);
-    if (T == 2) return q3::block_diag_rows_launch<2>(u, w, out, T, nb, bw, rows, stream);
-    if (T <= 4) return q3::block_diag_rows_launch<4>(u, w, out, T, nb, bw, rows, stream);
-    if (T <= 8) return q3::block_diag_rows_launch<8>(u, w, out, T, nb, bw, rows, stream);
-    return q3::block_diag_rows_launch<16>(u, w, out, T, nb, bw, rows, stream);
+    // tokens per block: all of them while they are few (a block reads its rows of w once), then groups, so that more warps
+    // hide each other's latencies; fewer where a row is long (8 tokens, 16 blocks of 128 x 512: 5.5 us with all, 3.4 with two)
+#define Q3_BDR(MT, WARPS) return q3::block_diag_rows_launch<MT, WARPS>(u, w, out, T, nb, bw, rows, stream)
+    if (rows <= 16) Q3_BDR(2, 2);
+    if (T == 1) Q3_BDR(1, 4);
+    if (T == 2 || (T <= 4 && bw > 256)) Q3_BDR(2, 4);
+    if (T <= 4) Q3_BDR(4, 4);
+    if (T <= 8 && bw > 256) Q3_BDR(2, 8);
+    if (T <= 8 || bw > 128) Q3_BDR(4, 8);
+    Q3_BDR(8, 8);
+#undef Q3_BDR
   }
   const int units = nb * rows;
   dim3 grid((units + q3::BD_WARPS - 1) / q3::BD_WARPS);
