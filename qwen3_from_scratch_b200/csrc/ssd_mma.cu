@@ -368,7 +368,8 @@ extern "C" int q3_ssd_scan_mma(const void* xbc, int ld, const void* proj, int ld
                                int num_slots, cudaStream_t stream) {
   if (T <= 0 || B <= 0) return 0;
   if (!q3_ssd_mma_takes(P, N) || H <= 0 || G <= 0 || H % G || !scratch) return Q3_ERR_SIZE;
-  if (ld % 8 || (H * P) % 8 || (uintptr_t)xbc % 16 || (uintptr_t)scratch % 16 || (uintptr_t)y % 8) return Q3_ERR_ALIGN;
+  if (ld % 8 || (H * P) % 8 || (uintptr_t)xbc % 16 || (uintptr_t)scratch % 16 || (uintptr_t)state % 16 || (uintptr_t)y % 8)
+    return Q3_ERR_ALIGN;
   if (N == 64)
     return q3::ssd_mma_launch<64, 64>(xbc, ld, proj, ld_proj, dt_col, dt_bias, A_log, Dp, state, scratch, q_start, slot_ids,
                                       y, B, max_q_len, H, G, num_slots, stream);

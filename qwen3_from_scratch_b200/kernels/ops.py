@@ -1887,7 +1887,8 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.
         _check("ssd_scan.scratch", scratch, torch.float32)
         if scratch.numel() < ssd_scratch_numel(T, num_seqs, heads, vdim, n_state):
             raise KernelError(f"ssd_scan: scratch of {scratch.numel()} floats for {T} tokens of {num_seqs} requests")
-    if chunked and kernel != "walk" and ssd_matrix_form(vdim, n_state) and ld % 8 == 0:
+    # (the matrix form renews the state 16 bytes at a time)
+    if chunked and kernel != "walk" and ssd_matrix_form(vdim, n_state) and ld % 8 == 0 and state.data_ptr() % 16 == 0:
         code = library().q3_ssd_scan_mma(xbc.data_ptr(), ld, proj.data_ptr(), proj.shape[1], int(dt_col),
                                          dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
                                          scratch.data_ptr(), q_start.data_ptr(), slot_ids.data_ptr(), y.data_ptr(), T,

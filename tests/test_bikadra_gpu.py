@@ -552,6 +552,31 @@ def test_state_space_walk_of_short_portions(H, P, N, G):
         close(states[0], S, "float32")
 
 
+def test_chunks_of_a_state_off_a_16_byte_boundary():
+    """The matrix form renews the state 16 bytes at a time; a state that begins elsewhere goes to the walk by chunks, whose
+    result agrees, and the matrix form's own entry refuses it."""
+    from qwen3_from_scratch_b200.kernels import ops
+    H, P, N, G, T = 2, 64, 64, 1, 300
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    xbc, proj, s0 = r(T, H * P + 2 * G * N).to(torch.bfloat16), r(T, H).to(torch.bfloat16), r(2, H, N, P)
+    consts, scratch, status = (r(H), r(H), r(H)), torch.empty(ops.ssd_scratch_numel(T, 1, H, P, N), device="cuda"), i32([0])
+    shifted = torch.empty(s0.numel() + 1, device="cuda")[1:].view(s0.shape).copy_(s0)
+    results = []
+    for state in (s0.clone(), shifted):
+        y = torch.full((T, H * P), float("nan"), device="cuda")
+        ops.ssd_scan(xbc, proj, 0, *consts, state, i32([0, T]), i32([1]), 1, y, H, P, N, G, status, max_q_len=T, scratch=scratch)
+        results.append((y, state))
+    assert int(status.item()) == 0 and torch.equal(shifted[0], s0[0])
+    for a, b in zip(*results):
+        close(b, a, "float32")
+    code = ops.library().q3_ssd_scan_mma(
+        xbc.data_ptr(), xbc.shape[1], proj.data_ptr(), H, 0, *(t.data_ptr() for t in consts), shifted.data_ptr(), scratch.data_ptr(),
+        i32([0, T]).data_ptr(), i32([1]).data_ptr(), results[0][0].data_ptr(), T, 1, T, H, P, N, G, 2, torch.cuda.current_stream().cuda_stream)
+    assert code == -3
+
+
 def test_matrix_form_sums_log_decays_in_the_order_of_the_tokens():
     """What a chunk leaves depends on differences of the running sums of its log-decays; summed token by token such a
     difference carries only the roundings of the steps between.  64 heads of 64 x 128, 300 tokens, decays of about one half
