@@ -21,9 +21,11 @@ constexpr int GF_LANE = 8;    // values of k of a lane at a time
 
 // ---------------------------------------------------------------- tiles
 // 64 x 64 outputs per block, four groups of 64 threads; group g walks over its chains (s, l) with 8 x 8 outputs per thread
-// and the four partial sums meet in shared memory.  Bound by the FMA pipe: 64 FMA per four 16-byte shared-memory reads.
-// The split over K inside the block gives a narrow product (N = 1,024 and 500 rows: 144 tiles of 64 x 64) a block on
-// every SM with eight warps of 8 x 8 register tiles, which tiles of 128 x 128 (32 blocks) could not.
+// and the four partial sums meet in shared memory (64 FMA per four 16-byte shared-memory reads).  The split over K inside
+// the block gives a narrow product more blocks than wider tiles would (N = 1,024 and 500 rows: 128 tiles of 64 x 64, with
+// eight warps each, against 32 of 128 x 128 for 148 SMs).  The FMA pipe is busy half of the time (513 x 4,096 x 1,024: 139.8 us,
+// 31 of 74 TFLOP/s): register-bank conflicts of 128 accumulators and the start of each tile, which nothing covers with one
+// block per SM, take the rest.
 constexpr int GF_T = 64, GF_GROUPS = 4, GF_GROUP_THREADS = 64, GF_THREADS = GF_GROUPS * GF_GROUP_THREADS, GF_STAGES = 3;
 constexpr int GF_STAGE_BYTES = 2 * GF_T * 128;                            // 64 rows of A, 64 of W, 32 values of k each
 constexpr int GF_RED_PITCH = GF_T + 8;                                    // floats: a thread's rows fall on different banks

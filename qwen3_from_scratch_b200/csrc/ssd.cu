@@ -28,26 +28,11 @@ __device__ __forceinline__ float ssd_update(float log_a, float a, float S, float
   return fmaf(a, S, b);
 }
 
-// SSD_PER values of row[col ..] as floats; VEC: bfloat16 with col a multiple of 8 and an aligned row (two 16-byte loads).
-template <typename T, bool VEC>
+// SSD_PER values of row[col ..] as floats, zeros beyond the first `live`.
+template <typename T>
 __device__ __forceinline__ void ssd_load16(const T* __restrict__ row, int col, int live, float (&v)[SSD_PER]) {
-  if constexpr (VEC) {
-    if (live <= 0) {  // a lane beyond the last state (the lanes are a power of two): nothing of its own to read
 #pragma unroll
-      for (int i = 0; i < SSD_PER; ++i) v[i] = 0.f;
-      return;
-    }
-    const uint4 lo = *reinterpret_cast<const uint4*>(row + col), hi = *reinterpret_cast<const uint4*>(row + col + 8);
-    const uint32_t wds[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[2 * i] = __uint_as_float(wds[i] << 16);
-      v[2 * i + 1] = __uint_as_float(wds[i] & 0xffff0000u);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < SSD_PER; ++i) v[i] = i < live ? to_float(row[col + i]) : 0.f;
-  }
+  for (int i = 0; i < SSD_PER; ++i) v[i] = i < live ? to_float(row[col + i]) : 0.f;
 }
 
 // A group of L lanes (a power of two, 16 states each) per (head, PP channels).  MODE 0: a request's whole portion from
@@ -57,7 +42,7 @@ __device__ __forceinline__ void ssd_load16(const T* __restrict__ row, int col, i
 // the threads (so that a chunk's state comes and goes in 16-byte pieces of whole lines), then H decay products
 // (padded to a multiple of four):
 // `record_floats` floats; chunk j of request b is record q_start[b] / SSD_CHUNK + b + j.
-// U (VEC only): tokens whose inputs are asked for together.
+// VEC: bfloat16, B and C of a lane in two 16-byte loads each.  U (VEC only): tokens whose inputs are asked for together.
 template <typename T, int PP, bool VEC, int MODE, int U>
 __global__ void __launch_bounds__(128)
 ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, int ld_proj, int dt_col,
@@ -178,8 +163,8 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
     const float a = exact ? expf(log_a) : __expf(log_a);
     log_total += log_a;
     float Bv[SSD_PER], Cv[SSD_PER], x[PP];
-    ssd_load16<T, VEC>(row, b_col, states, Bv);
-    if (MODE != 1) ssd_load16<T, VEC>(row, c_col, states, Cv);
+    ssd_load16(row, b_col, states, Bv);
+    if (MODE != 1) ssd_load16(row, c_col, states, Cv);
 #pragma unroll
     for (int c = 0; c < PP; ++c) x[c] = to_float(row[x_col + c]);
 #pragma unroll
@@ -188,7 +173,7 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ld, const T* __restrict__ proj, i
       float part = 0.f;
 #pragma unroll
       for (int i = 0; i < SSD_PER; ++i) {
-        if (VEC || i < states) {
+        if (i < states) {
           S[c][i] = ssd_update(log_a, a, S[c][i], sx * Bv[i], exact);
           if (MODE != 1) part = fmaf(S[c][i], Cv[i], part);
         }
