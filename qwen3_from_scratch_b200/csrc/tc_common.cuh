@@ -318,6 +318,16 @@ static int cached_map(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t
   const MapKey key{ptr, rows, cols, box_rows};
   uint64_t h = (uint64_t)(uintptr_t)ptr * 0x9E3779B97F4A7C15ull ^ (rows * 0xBF58476D1CE4E5B9ull) ^ (cols << 7) ^ box_rows;
   const int slot = (int)((h >> 32) % SLOTS);
+  // host threads share the slots: without the lock one could read a map while another writes it
+  static std::atomic_flag busy = ATOMIC_FLAG_INIT;
+  struct Lock {
+    std::atomic_flag& flag;
+    explicit Lock(std::atomic_flag& f) : flag(f) {
+      while (flag.test_and_set(std::memory_order_acquire)) {
+      }
+    }
+    ~Lock() { flag.clear(std::memory_order_release); }
+  } lock(busy);
   if (used[slot] && keys[slot] == key) {
     *map = maps[slot];
     return 0;

@@ -449,6 +449,43 @@ def test_gemm_tc_with_an_activation(M, N, K, activation):
     close(out, want, "bfloat16")
 
 
+def test_tcgen05_products_from_several_threads():
+    """Threads with streams of their own share the cache of tensor maps: each gets its own products right, among maps that
+    are made, replaced and read at the same time."""
+    import threading
+    g = torch.Generator().manual_seed(16)
+    jobs, wrong = [], []
+    for _ in range(4):
+        stream, products = torch.cuda.Stream(), []
+        for M in range(128, 448, 8):
+            x, w = dev(torch.randn(M, 64, generator=g).to(torch.bfloat16)), dev(torch.randn(136, 64, generator=g).to(torch.bfloat16))
+            out, want = torch.empty(M, 136, device="cuda", dtype=torch.bfloat16), torch.empty(M, 136, device="cuda", dtype=torch.bfloat16)
+            ops().gemm_tc(x, w, want, status())
+            products.append((x, w, out, want, M))
+        jobs.append((stream, products, status()))
+    torch.cuda.synchronize()
+    launch = ops().library()._lib.q3_gemm_tc
+
+    def work(stream, products, st):
+        with torch.cuda.stream(stream):  # (the thread's first use of the device)
+            st.zero_()
+        for _ in range(40):
+            for x, w, out, _, M in products:
+                code = launch(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, 136, 64, 136, 0, 0, st.data_ptr(), stream.cuda_stream)
+                if code:
+                    wrong.append((M, code))
+
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong
+    for _, products, st in jobs:
+        assert int(st.item()) == 0 and all(torch.equal(out, want) for _, _, out, want, _ in products)
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 16, 17])
 @pytest.mark.parametrize("nb,rows,bw", [(8, 512, 256), (3, 16, 8), (5, 48, 136), (2, 24, 40), (2, 32, 12)])
 def test_block_diag(T, nb, rows, bw):
