@@ -27,6 +27,22 @@ __device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& hi, __nv_bflo
   lo = __float2bfloat16_rn(v - __bfloat162float(hi));
 }
 
+// Four neighbouring values, as 8 bytes of upper and 8 of lower halves.
+__device__ __forceinline__ void split_bf16x4(float4 v, uint2& hi, uint2& lo) {
+  const float vv[4] = {v.x, v.y, v.z, v.w};
+  __nv_bfloat16 h[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) split_bf16(vv[i], h[i], l[i]);
+  hi = make_uint2(pack_bf16(__bfloat162float(h[0]), __bfloat162float(h[1])), pack_bf16(__bfloat162float(h[2]), __bfloat162float(h[3])));
+  lo = make_uint2(pack_bf16(__bfloat162float(l[0]), __bfloat162float(l[1])), pack_bf16(__bfloat162float(l[2]), __bfloat162float(l[3])));
+}
+// 16 bytes into shared memory, or zeros.
+__device__ __forceinline__ void sm_copy16(void* dst, const void* src, bool in) {
+  const int n = in ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n)
+               : "memory");
+}
+
 // What both kernels do first: the chunk's rows of x (this head's P channels), B and C (its group's N values) into
 // shared memory as [SM_Q][P + 8] and [SM_Q][N + 8], zero beyond the chunk's end; step sizes and the inclusive sums of
 // the log-decays (a row beyond the end has step 0 and decay 1: it changes nothing).
@@ -35,24 +51,20 @@ __device__ __forceinline__ void load_chunk(const __nv_bfloat16* __restrict__ xbc
                                            int ld_proj, int dt_col, int h, int g, int G, int inner, float rate, float db,
                                            int t0, int len, __nv_bfloat16* xs, __nv_bfloat16* bs, __nv_bfloat16* cs,
                                            float* step_s, float* cum_s) {
+  // every copy is on its way before anything waits: the block's time is latencies, not bytes
   constexpr int PX = P + 8, PN = N + 8;
+  const __nv_bfloat16* const rows = xbc + (size_t)t0 * ld;
   for (int i = threadIdx.x; i < SM_Q * (P / 8); i += blockDim.x) {
     const int t = i / (P / 8), c = i % (P / 8);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (t < len) v = *reinterpret_cast<const uint4*>(xbc + (size_t)(t0 + t) * ld + h * P + c * 8);
-    *reinterpret_cast<uint4*>(xs + t * PX + c * 8) = v;
+    sm_copy16(xs + t * PX + c * 8, rows + (t < len ? (size_t)t * ld + h * P + c * 8 : 0), t < len);
   }
   for (int i = threadIdx.x; i < SM_Q * (N / 8); i += blockDim.x) {
     const int t = i / (N / 8), c = i % (N / 8);
-    uint4 vb = make_uint4(0, 0, 0, 0), vc = make_uint4(0, 0, 0, 0);
-    if (t < len) {
-      const __nv_bfloat16* row = xbc + (size_t)(t0 + t) * ld + inner + g * N + c * 8;
-      vb = *reinterpret_cast<const uint4*>(row);
-      if (WANT_C) vc = *reinterpret_cast<const uint4*>(row + (size_t)G * N);
-    }
-    *reinterpret_cast<uint4*>(bs + t * PN + c * 8) = vb;
-    if (WANT_C) *reinterpret_cast<uint4*>(cs + t * PN + c * 8) = vc;
+    const __nv_bfloat16* row = rows + (t < len ? (size_t)t * ld + inner + g * N + c * 8 : 0);
+    sm_copy16(bs + t * PN + c * 8, row, t < len);
+    if (WANT_C) sm_copy16(cs + t * PN + c * 8, row + (t < len ? (size_t)G * N : 0), t < len);
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
   if (threadIdx.x < SM_Q) {
     const int t = threadIdx.x;
     float step = 0.f;
@@ -85,7 +97,13 @@ __device__ __forceinline__ void load_chunk(const __nv_bfloat16* __restrict__ xbc
       }
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+}
+
+// bfloat16 values of the output kernel's shared memory: x, then B and C or the state's halves
+__host__ __device__ constexpr int ssd_output_halves(int P, int N) {
+  return SM_Q * (P + 8) + (2 * SM_Q * (N + 8) > 2 * N * (P + 8) ? 2 * SM_Q * (N + 8) : 2 * N * (P + 8));
 }
 
 // grid (requests, chunks, heads), 128 threads.  Leaves in the chunk's record: reached[h][n][p] =
@@ -115,10 +133,19 @@ ssd_chunk_state_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __nv
   load_chunk<P, N, false>(xbc, ld, proj, ld_proj, dt_col, h, g, G, inner, -expf(A_log[h]), dt_bias[h], t0, len, xs, bs,
                           nullptr, step_s, cum_s);
   const float last = cum_s[SM_Q - 1];
-  for (int i = threadIdx.x; i < SM_Q * P; i += blockDim.x) {
-    const int s = i / P, p = i % P;
+  for (int i = threadIdx.x; i < SM_Q * P / 8; i += blockDim.x) {
+    const int s = i / (P / 8), at = s * PX + (i % (P / 8)) * 8;
     const float w = __expf(last - cum_s[s]) * step_s[s];
-    split_bf16(w * __bfloat162float(xs[s * PX + p]), xw_hi[s * PX + p], xw_lo[s * PX + p]);
+    const uint4 x8 = *reinterpret_cast<const uint4*>(xs + at);
+    const uint32_t xv[4] = {x8.x, x8.y, x8.z, x8.w};
+    uint2 hi[2], lo[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      split_bf16x4(make_float4(w * __uint_as_float(xv[2 * k] << 16), w * __uint_as_float(xv[2 * k] & 0xffff0000u),
+                               w * __uint_as_float(xv[2 * k + 1] << 16), w * __uint_as_float(xv[2 * k + 1] & 0xffff0000u)),
+                   hi[k], lo[k]);
+    *reinterpret_cast<uint4*>(xw_hi + at) = make_uint4(hi[0].x, hi[0].y, hi[1].x, hi[1].y);
+    *reinterpret_cast<uint4*>(xw_lo + at) = make_uint4(lo[0].x, lo[0].y, lo[1].x, lo[1].y);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tid4 = lane & 3;
@@ -203,8 +230,12 @@ ssd_chunk_carry_kernel(float* __restrict__ scratch, float* __restrict__ state, c
 }
 
 // grid (requests, chunks, heads), 128 threads: warp w owns the chunk's rows 16 w .. 16 w + 15.
+// A block is a chain of latencies (rows, decays, products, state, products), so as many as possible share an SM: the state
+// takes the place of B and C once their product is in registers (47 KB, four blocks; two while each had its own), and is
+// asked into L2 before the block waits for anything.  (32 chunks of 64 heads of 64 x 128 inside a step: 87 us before, 59 now, for
+// 115 MB; the states' kernel, whose weighted x is split eight values at a time, 39 and 30.)
 template <int P, int N>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 4)
 ssd_chunk_output_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __nv_bfloat16* __restrict__ proj, int ld_proj,
                         int dt_col, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                         const float* __restrict__ Dp, const float* __restrict__ scratch, const int* __restrict__ q_start,
@@ -215,9 +246,9 @@ ssd_chunk_output_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __n
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(sm_raw);  // [SM_Q][PX]
   __nv_bfloat16* bs = xs + SM_Q * PX;                            // [SM_Q][PN]
   __nv_bfloat16* cs = bs + SM_Q * PN;                            // [SM_Q][PN]
-  __nv_bfloat16* s_hi = cs + SM_Q * PN;                          // [N][PX]: the state the chunk starts from
+  __nv_bfloat16* s_hi = bs;                                      // [N][PX]: the state the chunk starts from, after B and C
   __nv_bfloat16* s_lo = s_hi + N * PX;
-  float* step_s = reinterpret_cast<float*>(s_lo + N * PX);
+  float* step_s = reinterpret_cast<float*>(xs + ssd_output_halves(P, N));
   float* cum_s = step_s + SM_Q;
   pdl_wait();
   pdl_launch_dependents();
@@ -233,13 +264,7 @@ ssd_chunk_output_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __n
     return;
   }
   const float* rec = scratch + (size_t)(start / SM_Q + b + blockIdx.y) * record_floats + (size_t)h * N * P;
-  for (int i = threadIdx.x; i < N * P / 4; i += blockDim.x) {
-    const float4 v = reinterpret_cast<const float4*>(rec)[i];
-    const int n = (4 * i) / P, p = (4 * i) % P;
-    const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) split_bf16(vv[k], s_hi[n * PX + p + k], s_lo[n * PX + p + k]);
-  }
+  for (int i = threadIdx.x; i < N * P / 32; i += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + i * 32));
   load_chunk<P, N, true>(xbc, ld, proj, ld_proj, dt_col, h, g, G, inner, -expf(A_log[h]), dt_bias[h], t0, len, xs, bs, cs,
                          step_s, cum_s);
   // this warp's rows of C as A fragments, for G = C B^T and for C S_in
@@ -279,12 +304,9 @@ ssd_chunk_output_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __n
     m_lo[kk][half + 1] = pack_bf16(__bfloat162float(lo[2]), __bfloat162float(lo[3]));
   }
   // y = M X + e^{cum_t} (C S_in) + D x
-  float acc[P / 8][4], z[P / 8][4];
+  float acc[P / 8][4];
 #pragma unroll
-  for (int i = 0; i < P / 8; ++i) {
-    acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    z[i][0] = z[i][1] = z[i][2] = z[i][3] = 0.f;
-  }
+  for (int i = 0; i < P / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 #pragma unroll
   for (int kk = 0; kk < SM_Q / 16; ++kk)
 #pragma unroll
@@ -296,6 +318,27 @@ ssd_chunk_output_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __n
       mma_bf16(acc[2 * dt], m_lo[kk], vb[0], vb[1]);
       mma_bf16(acc[2 * dt + 1], m_lo[kk], vb[2], vb[3]);
     }
+  __syncthreads();  // every warp is done with B and C
+  constexpr int SBATCH = 8;
+  static_assert(N * P / 4 % (128 * SBATCH) == 0, "whole batches");
+#pragma unroll 1
+  for (int i0 = threadIdx.x; i0 < N * P / 4; i0 += 128 * SBATCH) {
+    float4 v[SBATCH];
+#pragma unroll
+    for (int k = 0; k < SBATCH; ++k) v[k] = reinterpret_cast<const float4*>(rec)[i0 + 128 * k];
+#pragma unroll
+    for (int k = 0; k < SBATCH; ++k) {
+      const int at = (i0 + 128 * k) / (P / 4) * PX + (i0 + 128 * k) % (P / 4) * 4;
+      uint2 hi, lo;
+      split_bf16x4(v[k], hi, lo);
+      *reinterpret_cast<uint2*>(s_hi + at) = hi;
+      *reinterpret_cast<uint2*>(s_lo + at) = lo;
+    }
+  }
+  __syncthreads();
+  float z[P / 8][4];
+#pragma unroll
+  for (int i = 0; i < P / 8; ++i) z[i][0] = z[i][1] = z[i][2] = z[i][3] = 0.f;
 #pragma unroll
   for (int ks = 0; ks < N / 16; ++ks)
 #pragma unroll
@@ -333,7 +376,7 @@ static int ssd_mma_launch(const void* xbc, int ld, const void* proj, int ld_proj
   using bf16 = __nv_bfloat16;
   constexpr int PX = P + 8, PN = N + 8;
   const size_t smem1 = (size_t)(3 * SM_Q * PX + SM_Q * PN) * sizeof(bf16) + 2 * SM_Q * sizeof(float);
-  const size_t smem2 = (size_t)(SM_Q * PX + 2 * SM_Q * PN + 2 * N * PX) * sizeof(bf16) + 2 * SM_Q * sizeof(float);
+  const size_t smem2 = (size_t)ssd_output_halves(P, N) * sizeof(bf16) + 2 * SM_Q * sizeof(float);
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(ssd_chunk_state_kernel<P, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
