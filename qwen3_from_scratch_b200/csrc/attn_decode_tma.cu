@@ -6,6 +6,10 @@
 // tile: the loader runs up to a ring of 16-key tiles (64 KB per block at D = 128) ahead, which is what
 // a bandwidth-bound kernel wants, and the consumers issue no copy instructions at all.
 //
+// SIGMOID: the weights of attn_sigmoid.cu (sigmoid(s * scale + head_bias[h]), not normalised; the finished row times
+// gate[t, h]): no maximum, no denominator, and the ranges' partial sums are plain sums.  (Eight requests at 2,048 tokens, 16 heads over 8 of
+// 128, inside a step: 16 us where the cp.async kernel took 29, for 10 of cache bytes.)
+//
 // Takes D = 64 or 128 and page sizes that are multiples of 16 (a 16-key tile then lies in one
 // page); everything else goes to attn_decode.cu.  Mbarrier waits are bounded (tc_common.cuh).
 #include "attn_mma.cuh"
@@ -13,6 +17,8 @@
 
 extern "C" int q3_attn_combine(const float* partial, void* out, const int* q_start, int B, int Hq, int D,
                                int num_splits, cudaStream_t stream);
+extern "C" int q3_sum_gate(const float* partial, const float* gate, const int* q_start, void* out, int B, int Hq, int D,
+                           int num_splits, cudaStream_t stream);
 
 namespace q3 {
 
@@ -107,6 +113,8 @@ struct DecodeQkv {
   int write_kv;              // 0: another layer wrote this cache; only the query is made
   int angles_early;          // cos_sin is older than the launch before this one
   const float* sink;         // float32 [Hq]: exp(sink) joins the denominator; or null
+  const float* head_bias;    // SIGMOID: float32 [Hq] or null
+  const float* gate;         // SIGMOID: float32 [T, Hq] or null
   int beside;                // the launch before this one is the portions' attention of the same step, see below
 };
 
@@ -124,7 +132,7 @@ struct DecodeQkv {
 // (smaller blocks, see DecodeTmaBlock) are for a grid of several waves, where more blocks per SM in different
 // stages of their lives keep the SM's stream over the cache going
 // (figures: profiles/attn_decode_tma__decode_b8_ctx4096.md).
-template <int D, int BLOCKS>
+template <int D, int BLOCKS, bool SIGMOID = false>
 __global__ void __launch_bounds__(DecodeTmaBlock<BLOCKS>::THREADS, BLOCKS)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ out,
@@ -274,6 +282,12 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt)
       ldmatrix_x4(qa[kt], q_s + ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + kt * 16 + (lane >> 4) * 8);
+    float bias_log2[2] = {0.f, 0.f};  // SIGMOID: of the rows gid and gid + 8, in the units of the base-2 exponential
+    if (SIGMOID && fq.head_bias != nullptr) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        if (gid + 8 * r < g) bias_log2[r] = fq.head_bias[hk * g + gid + 8 * r] * 1.4426950408889634f;
+    }
     bool ok = true;
     for (int i = warp; i < count; i += DT_CONSUMERS) {
       const int s = i % DT_STAGES;
@@ -362,15 +376,23 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         mma_bf16(sc[0], qa[kt], kb[0], kb[1]);
         mma_bf16(sc[1], qa[kt], kb[2], kb[3]);
       }
+      if (SIGMOID) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            sc[nt][j] = __fdividef(1.0f, 1.0f + ex2_approx(-fmaf(sc[nt][j], scale_log2, bias_log2[j >> 1])));
+      }
       if (edge) {
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int n = base_n + nt * 8 + 2 * tid4 + (j & 1);
-            if (n < lo || n > pos) sc[nt][j] = -INFINITY;
+            if (n < lo || n > pos) sc[nt][j] = SIGMOID ? 0.f : -INFINITY;
           }
       }
+      if (!SIGMOID) {
       float mx[2];
       mx[0] = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
       mx[1] = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
@@ -405,6 +427,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           sc[nt][2 * r + 1] = p1;
           l[r] += p0 + p1;
         }
+      }  // softmax
       uint32_t pa[4];
       pa[0] = pack_bf16(sc[0][0], sc[0][1]);
       pa[1] = pack_bf16(sc[0][2], sc[0][3]);
@@ -457,7 +480,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
     for (int w = 0; w < DT_CONSUMERS; ++w) big = fmaxf(big, merge[((size_t)w * 16 + r) * (D + 2) + D]);
     float acc = 0.f, den = 0.f;
-    if (big != -INFINITY) {
+    if (SIGMOID) {
+#pragma unroll
+      for (int w = 0; w < DT_CONSUMERS; ++w) acc += merge[((size_t)w * 16 + r) * (D + 2) + d];
+    } else if (big != -INFINITY) {
 #pragma unroll
       for (int w = 0; w < DT_CONSUMERS; ++w) {
         const float* row = merge + ((size_t)w * 16 + r) * (D + 2);
@@ -474,7 +500,11 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       den = fmaf(den, keep, exp2f(s2 - top));
       big = top;
     }
-    if (num_splits == 1) {
+    if (SIGMOID) {
+      const size_t at = (size_t)tq * Hq + head;
+      if (num_splits == 1) out[at * D + d] = __float2bfloat16_rn(acc * (fq.gate != nullptr ? fq.gate[at] : 1.f));
+      else partial[(((size_t)b * num_splits + split) * Hq + head) * D + d] = acc;
+    } else if (num_splits == 1) {
       out[((size_t)tq * Hq + head) * D + d] = __float2bfloat16_rn(den > 0.f ? acc / den : 0.f);
     } else {
       float* p = partial + (((size_t)b * Hq + head) * num_splits + split) * (D + 2);
@@ -491,20 +521,20 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   }
 }
 
-template <int D>
+template <int D, bool SIGMOID = false>
 static int attn_decode_tma_launch(const void* q, const void* k_pages, const void* v_pages, void* out, float* partial,
                                   const int* q_start, const int* kv_len, const int* block_table, int table_stride,
                                   int page_size, int num_pages, int B, int Hq, int Hkv, float scale, int window,
                                   int num_splits, int* status, cudaStream_t stream, DecodeQkv fq = DecodeQkv{}) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, 2, SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)DecodeTmaShape<D, 2>::SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, 3, SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)DecodeTmaShape<D, 3>::SMEM_BYTES);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(attn_decode_tma_kernel<D, 4, SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)DecodeTmaShape<D, 4>::SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     configured = true;
@@ -520,7 +550,7 @@ static int attn_decode_tma_launch(const void* q, const void* k_pages, const void
   // two blocks per SM where the grid fits them, three where it fits those, four for a grid of several waves
   const int per_sm = blocks <= 2LL * sm_count() ? 2 : blocks <= 3LL * sm_count() ? 3 : 4;
 #define Q3_DT_LAUNCH(BL)                                                                                              \
-  q3::launch(attn_decode_tma_kernel<D, BL>, grid, dim3(DecodeTmaBlock<BL>::THREADS), DecodeTmaShape<D, BL>::SMEM_BYTES,  \
+  q3::launch(attn_decode_tma_kernel<D, BL, SIGMOID>, grid, dim3(DecodeTmaBlock<BL>::THREADS), DecodeTmaShape<D, BL>::SMEM_BYTES,  \
              stream, map_k, map_v, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, partial, q_start, kv_len, block_table, \
              table_stride, page_size, num_pages, Hq, Hkv, scale * 1.4426950408889634f, window, num_splits, status, fq)
   if (per_sm == 2) Q3_DT_LAUNCH(2);
@@ -529,6 +559,7 @@ static int attn_decode_tma_launch(const void* q, const void* k_pages, const void
 #undef Q3_DT_LAUNCH
   code = launch_status();
   if (code != 0 || num_splits == 1) return code;
+  if (SIGMOID) return q3_sum_gate(partial, fq.gate, q_start, out, B, Hq, D, num_splits, stream);
   return q3_attn_combine(partial, out, q_start, B, Hq, D, num_splits, stream);
 }
 
@@ -575,6 +606,29 @@ extern "C" int q3_attn_decode_tma_beside(const void* q, const void* k_pages, con
                                           page_size, num_pages, B, Hq, Hkv, scale, window, num_splits, status, stream, fq);
   return q3::attn_decode_tma_launch<128>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride,
                                          page_size, num_pages, B, Hq, Hkv, scale, window, num_splits, status, stream, fq);
+}
+
+// The same with sigmoid weights (see attn_sigmoid.cu): head_bias float32 [Hq] or null, gate float32 [T, Hq] or null;
+// partial: float32 [B, num_splits, Hq, D], needed for more than one range.
+extern "C" int q3_attn_sigmoid_decode_tma(const void* q, const void* k_pages, const void* v_pages, void* out, float* partial,
+                                          const float* head_bias, const float* gate, const int* q_start, const int* kv_len,
+                                          const int* block_table, int table_stride, int page_size, int num_pages, int B,
+                                          int Hq, int Hkv, int D, float scale, int num_splits, int* status,
+                                          cudaStream_t stream) {
+  if (B <= 0) return 0;
+  if (Hkv <= 0 || Hq % Hkv || Hq / Hkv > 16 || (D != 64 && D != 128) || page_size <= 0 || page_size % 16 ||
+      num_splits < 1 || table_stride <= 0 || B > 65535 || Hkv > 65535)
+    return Q3_ERR_SIZE;
+  if (num_splits > 1 && !partial) return Q3_ERR_SCRATCH;
+  if ((uintptr_t)q % 16 || (uintptr_t)k_pages % 16 || (uintptr_t)v_pages % 16 || (uintptr_t)out % 4) return Q3_ERR_ALIGN;
+  q3::DecodeQkv fq{};
+  fq.head_bias = head_bias;
+  fq.gate = gate;
+  if (D == 64)
+    return q3::attn_decode_tma_launch<64, true>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride,
+                                                page_size, num_pages, B, Hq, Hkv, scale, 0, num_splits, status, stream, fq);
+  return q3::attn_decode_tma_launch<128, true>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride,
+                                               page_size, num_pages, B, Hq, Hkv, scale, 0, num_splits, status, stream, fq);
 }
 
 // The same with a sink (float32 [Hq]): exp(sink) joins the softmax's denominator.  The scale must be positive.

@@ -71,6 +71,9 @@ _SIGNATURES = {
     "q3_attn_decode_tma_beside": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                                   _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int,
                                   _c_void_p, _c_void_p],
+    "q3_attn_sigmoid_decode_tma": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
+                                   _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
+                                   _c_int, _c_void_p, _c_void_p],
     "q3_attn_decode_tma_qkv": [_c_void_p, _c_void_p, _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p,
                                _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                _c_int, _c_float, _c_int, _c_int, _c_void_p, _c_void_p],
@@ -1567,9 +1570,10 @@ def attn_sigmoid_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                      head_bias: Optional[torch.Tensor], gate: Optional[torch.Tensor], q_start: torch.Tensor,
                      kv_len: torch.Tensor, block_table: torch.Tensor, num_seqs: int, max_q_len: int, scale: float,
                      status: torch.Tensor, decode: bool = False, num_splits: int = 1,
-                     partial: Optional[torch.Tensor] = None) -> None:
+                     partial: Optional[torch.Tensor] = None, loader: str = "cp_async") -> None:
     """The tensor-core kernel for ``num_seqs`` rows of the batch (q_start has num_seqs + 1 entries): portions of
-    any length, or with ``decode`` one token per row, the keys cut into ``num_splits`` ranges."""
+    any length, or with ``decode`` one token per row, the keys cut into ``num_splits`` ranges (``loader="tma"``: by the
+    kernel of ``attn_decode`` with that loader, where ``decode_tma_takes`` the shape)."""
     T, Hq, D, num_pages, Hkv, page_size = _attn_common("attn_sigmoid_mma", q, k_pages, v_pages, out, q_start, kv_len,
                                                         block_table)
     if q_start.numel() < num_seqs + (0 if decode else 1) or kv_len.numel() < num_seqs or block_table.shape[0] < num_seqs:
@@ -1585,6 +1589,15 @@ def attn_sigmoid_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         _check("attn_sigmoid_mma.partial", partial, torch.float32)
         if partial.numel() < num_seqs * num_splits * Hq * D:
             raise KernelError(f"attn_sigmoid_mma: scratch of {partial.numel()} floats for {num_seqs} x {num_splits} ranges")
+    if loader == "tma":
+        if not decode:
+            raise KernelError("attn_sigmoid_mma: the TMA loader is for single tokens")
+        code = library().q3_attn_sigmoid_decode_tma(
+            q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(), _ptr(partial), _ptr(head_bias), _ptr(gate),
+            q_start.data_ptr(), kv_len.data_ptr(), block_table.data_ptr(), block_table.shape[1], page_size, num_pages, num_seqs,
+            Hq, Hkv, D, float(scale), int(num_splits), status.data_ptr(), _stream())
+        _done("attn_sigmoid_mma", code, f"heads {Hq}/{Hkv}, head_dim {D}, page {page_size}, loader tma")
+        return
     code = library().q3_attn_sigmoid_mma(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(),
                                          _ptr(partial), _ptr(head_bias), _ptr(gate), q_start.data_ptr(), kv_len.data_ptr(),
                                          block_table.data_ptr(), block_table.shape[1], page_size, num_pages, num_seqs,
@@ -1621,9 +1634,10 @@ def sigmoid_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
                       num_decode: int, max_q_len: int, max_kv_len: int, scale: float, status: torch.Tensor,
                       partial: Optional[torch.Tensor] = None, kernel: str = "auto") -> None:
     """Causal attention with sigmoid weights of a mixed batch over the pages (see ``attn_sigmoid``): rows
-    [0, num_decode) bring one token each and go to the decode form of the tensor-core kernel, the rest to its
+    [0, num_decode) bring one token each and go to the decode form of the tensor-core kernel (with the TMA loader for heads
+    of 64 or 128 and pages in multiples of 16), the rest to its
     portion form, or for heads of 64 or 128 and pages of 8 to 64 tokens to the tcgen05 kernel (``kernel="mma"``
-    keeps them on mma.sync); float32, shapes it refuses and ``kernel="plain"`` go to the plain kernel."""
+    keeps both on mma.sync and cp.async); float32, shapes it refuses and ``kernel="plain"`` go to the plain kernel."""
     T, Hq, D = q.shape
     Hkv = k_pages.shape[1]
     if block_table.dim() != 2 or max_kv_len > block_table.shape[1] * k_pages.shape[2]:
@@ -1634,11 +1648,14 @@ def sigmoid_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         return
     decode = num_decode if Hq // Hkv <= 16 else 0  # a wider group's single tokens run as portions of one
     if decode > 0:
-        splits = sigmoid_decode_splits(decode, Hkv, max_kv_len)
+        # the TMA loader where it takes the shape, with the ranges of the softmax's decode kernel (the same blocks and bytes)
+        tma = kernel != "mma" and decode_tma_takes(D, k_pages.shape[2])
+        splits = (decode_splits(decode, Hkv, max_kv_len, 0, D, blocks_per_sm=3, wide_blocks_per_sm=4) if tma
+                  else sigmoid_decode_splits(decode, Hkv, max_kv_len))
         if partial is None or partial.numel() < decode * splits * Hq * D:
             splits = 1 if partial is None else max(1, partial.numel() // (decode * Hq * D))
         attn_sigmoid_mma(q, k_pages, v_pages, out, head_bias, gate, q_start, kv_len, block_table, decode, 1, scale,
-                         status, decode=True, num_splits=splits, partial=partial)
+                         status, decode=True, num_splits=splits, partial=partial, loader="tma" if tma else "cp_async")
     if num_seqs > decode:
         rest = (q_start[decode:], kv_len[decode:], block_table[decode:], num_seqs - decode, max_q_len, scale, status)
         if kernel != "mma" and max_q_len > 1 and attn_tc_takes(D, k_pages.shape[2], 0):

@@ -336,6 +336,43 @@ def test_tensor_core_sigmoid_attention_equals_the_plain_kernel(hq, hkv, d, page)
         assert float((got.float() - want.float()).abs().max()) <= 1.5e-2 * scale, (partial_floats, kernel)
 
 
+@pytest.mark.parametrize("hq,hkv,d,page,splits,shift", [(16, 8, 128, 16, 1, 0), (16, 8, 128, 32, 3, 0), (16, 1, 64, 16, 2, 1),
+                                                        (3, 3, 64, 48, 32, 0), (8, 2, 128, 16, 7, 1)])
+def test_single_tokens_with_sigmoid_weights_by_the_tma_loader(hq, hkv, d, page, splits, shift):
+    """Contexts around the edges of a tile of 16 keys, in one range and in more ranges than some have tiles, with NaN in the
+    slots behind them, with and without bias and gate, with scratch that begins off a 16-byte boundary, against the plain
+    kernel: both round the weights' sum to bfloat16 once, the fast one also each weight."""
+    from qwen3_from_scratch_b200.kernels import ops
+    g = torch.Generator().manual_seed(43)
+    kv_lens = [1, 15, 16, 17, 48, 49, 333, 1000] + [5 + i for i in range(40)]  # blocks enough for every compiled form
+    B = len(kv_lens)
+    pages_per = [-(-n // page) for n in kv_lens]
+    order, at = torch.randperm(sum(pages_per), generator=g).tolist(), 0
+    table = torch.full((B, max(pages_per)), -1, dtype=torch.int32)
+    pools = [torch.full((sum(pages_per), hkv, page, d), float("nan"), dtype=torch.bfloat16) for _ in range(2)]
+    for b, n in enumerate(kv_lens):
+        ids = order[at:at + pages_per[b]]
+        table[b, :len(ids)] = torch.tensor(ids, dtype=torch.int32)
+        at += len(ids)
+        for i, page_id in enumerate(ids):
+            live = min(page, n - i * page)
+            for pool in pools:
+                pool[page_id, :, :live] = torch.randn(hkv, live, d, generator=g).to(torch.bfloat16)
+    k_pages, v_pages = (pool.cuda() for pool in pools)
+    q = (2 * torch.randn(B, hq, d, generator=g)).to(torch.bfloat16).cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    status, table = torch.zeros(1, dtype=torch.int32, device="cuda"), table.cuda()
+    partial = torch.full((B * splits * hq * d + shift,), float("nan"), device="cuda")[shift:]
+    for bias, gate in ((torch.randn(hq, generator=g).cuda() - 3, torch.rand(B, hq, generator=g).cuda()), (None, None)):
+        want, got = torch.empty_like(q), torch.full_like(q, float("nan"))
+        ops.attn_sigmoid(q, k_pages, v_pages, want, bias, gate, i32(list(range(B + 1))), i32(kv_lens), i32(list(range(B))), table,
+                         d ** -0.5, status)
+        ops.attn_sigmoid_mma(q, k_pages, v_pages, got, bias, gate, i32(list(range(B + 1))), i32(kv_lens), table, B, 1, d ** -0.5,
+                             status, decode=True, num_splits=splits, partial=partial, loader="tma")
+        assert int(status.item()) == 0
+        assert float((got.float() - want.float()).abs().max()) <= 1.5e-2 * float(want.float().abs().max())
+
+
 # ---------------------------------------------------------------------- whole models
 def tolerance(dtype, cfg, w, seqs):
     """float32: the harness's bound.  bfloat16: three times what rounding alone does to these prompts in the plain
