@@ -115,17 +115,7 @@ struct DecodeQkv {
   const float* sink;         // float32 [Hq]: exp(sink) joins the denominator; or null
   const float* head_bias;    // SIGMOID: float32 [Hq] or null
   const float* gate;         // SIGMOID: float32 [T, Hq] or null
-  int beside;                // the launch before this one is the portions' attention of the same step, see below
 };
-
-// Beside the portions' attention (q3_attn_decode_tma_beside).  A step that has both runs the portions first; their blocks
-// leave SMs one by one (a portion's last query tile walks all of its keys, its first ones few), and neither kernel reads
-// what the other writes.  So this kernel then does not wait for the one before it when it starts: its blocks start once
-// every block of that kernel has passed its own wait (common.cuh: everything older is complete), take the places that the
-// short tiles give back and read while the long ones still multiply.  It waits at its end instead, before it lets the next
-// kernel go, so that the next one starts after both, as ever.  (23 requests of 200 to 1,500 tokens beside portions of 37, 411
-// and 700 after 512, 16 heads over 8 of 128: 28 + 25 us one after the other, 45 side by side; the step of 28 layers 3,189 and
-// 3,038 us.)
 
 // BLOCKS: blocks per SM the kernel is compiled for.  Three (128 registers) give a large grid half as many
 // places again as two; two (168 registers) are the faster code where the grid fits their places anyway; four
@@ -200,10 +190,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                           : (which == 2 && fq.angles_early && fq.cos_sin) ? fq.cos_sin + (size_t)tq * D : nullptr;
       if (base != nullptr) asm volatile("prefetch.global.L1 [%0];" ::"l"(base + line * 32));
     }
-    if (!fq.beside) {
-      pdl_wait();
-      pdl_launch_dependents();
-    }
+    pdl_wait();
+    pdl_launch_dependents();
     for (int e = threadIdx.x; e < 16 * CPR; e += DT_CONSUMERS * 32) {
       const int row = e / CPR, c = e % CPR;  // a row's CPR chunks of eight values sit in neighbouring lanes
       uint4 v = make_uint4(0, 0, 0, 0);
@@ -265,12 +253,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     // before that tile can be fetched while that kernel still runs
     const int early_tiles = min(count, max(0, pos / DT_KEYS - t_lo));
     issue(0, early_tiles);
-    if (fq.beside) {
-      asm volatile("fence.proxy.async.global;" ::: "memory");  // the newest tile: plain stores of an earlier kernel
-    } else {
-      pdl_wait();
-      pdl_launch_dependents();  // after the wait, as everywhere: the next kernel never starts before the one before this ended
-    }
+    pdl_wait();
+    pdl_launch_dependents();  // after the wait, as everywhere: the next kernel never starts before the one before this ended
     issue(early_tiles, count);
     if (!ok && lane == 0) {
       *abort_word = 1;
@@ -515,10 +499,6 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
     }
   }
-  if (fq.beside) {
-    pdl_wait();
-    pdl_launch_dependents();
-  }
 }
 
 template <int D, bool SIGMOID = false>
@@ -586,26 +566,6 @@ extern "C" int q3_attn_decode_tma(const void* q, const void* k_pages, const void
   return q3::attn_decode_tma_launch<128>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table,
                                          table_stride, page_size, num_pages, B, Hq, Hkv, scale, window, num_splits,
                                          status, stream);
-}
-
-// The same for a step that has portions of prompts too, launched directly after their attention on the same stream (which
-// must not write what this reads, nor read what this writes): the two run side by side, see DecodeQkv::beside.
-extern "C" int q3_attn_decode_tma_beside(const void* q, const void* k_pages, const void* v_pages, void* out, float* partial,
-                                         const int* q_start, const int* kv_len, const int* block_table, int table_stride,
-                                         int page_size, int num_pages, int B, int Hq, int Hkv, int D, float scale,
-                                         int window, int num_splits, int* status, cudaStream_t stream) {
-  if (B <= 0) return 0;
-  if (Hkv <= 0 || Hq % Hkv || Hq / Hkv > 16 || (D != 64 && D != 128) || page_size <= 0 || page_size % 16 ||
-      num_splits < 1 || table_stride <= 0 || B > 65535 || Hkv > 65535)
-    return Q3_ERR_SIZE;
-  if ((uintptr_t)q % 16 || (uintptr_t)k_pages % 16 || (uintptr_t)v_pages % 16) return Q3_ERR_ALIGN;
-  q3::DecodeQkv fq{};
-  fq.beside = 1;
-  if (D == 64)
-    return q3::attn_decode_tma_launch<64>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride,
-                                          page_size, num_pages, B, Hq, Hkv, scale, window, num_splits, status, stream, fq);
-  return q3::attn_decode_tma_launch<128>(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, table_stride,
-                                         page_size, num_pages, B, Hq, Hkv, scale, window, num_splits, status, stream, fq);
 }
 
 // The same with sigmoid weights (see attn_sigmoid.cu): head_bias float32 [Hq] or null, gate float32 [T, Hq] or null;

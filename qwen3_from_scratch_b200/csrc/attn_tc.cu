@@ -104,7 +104,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   if (row0 >= total_rows) return;  // before any barrier or allocation: the whole block leaves
   const int past = len - q_len;
   if (past < 0) {  // more new tokens than the request holds; also before any barrier or allocation
-    pdl_wait();    // (a kernel beside this one relies on the wait, see attn_decode_tma.cu)
     if (threadIdx.x == 0) atomicOr(status, Q3_STATUS_BAD_POSITION);
     return;
   }

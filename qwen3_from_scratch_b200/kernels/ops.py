@@ -68,9 +68,6 @@ _SIGNATURES = {
     "q3_attn_decode_tma": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                            _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int,
                            _c_void_p, _c_void_p],
-    "q3_attn_decode_tma_beside": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
-                                  _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int,
-                                  _c_void_p, _c_void_p],
     "q3_attn_sigmoid_decode_tma": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                                    _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
                                    _c_int, _c_void_p, _c_void_p],
@@ -1092,15 +1089,12 @@ def _attn_common(name, q, k_pages, v_pages, out, q_start, kv_len, block_table):
 def attn_decode(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor,
                 partial: Optional[torch.Tensor], q_start: torch.Tensor, kv_len: torch.Tensor,
                 block_table: torch.Tensor, num_seqs: int, scale: float, window: int, num_splits: int,
-                status: torch.Tensor, loader: str = "cp_async", raw_qkv=None, sink: Optional[torch.Tensor] = None,
-                beside: bool = False) -> None:
+                status: torch.Tensor, loader: str = "cp_async", raw_qkv=None, sink: Optional[torch.Tensor] = None) -> None:
     """Split-KV tensor-core attention for the first ``num_seqs`` rows, one query token each.
     ``raw_qkv = (qkv, q_weight, k_weight, eps, cos_sin, write_kv)`` (TMA loader only): ``q`` only gives the
     shape; the kernel norms and rotates the query from the raw projection ``qkv[T, (Hq + 2 Hkv) D]`` itself
     and makes, stores and uses the new key and value (the work of ``qkv_post`` for these tokens).
     ``sink`` (float32 [Hq], TMA loader only, a positive scale): exp(sink) joins the softmax's denominator.
-    ``beside`` (TMA loader, neither of the two above): the launch before this one is the attention of the same step's
-    portions (``attn_tc`` on other rows); the two run side by side.
     ``loader``: ``"cp_async"`` (every warp copies its own tiles) or ``"tma"`` (a loader warp feeds a
     ring of stages through TMA; head size 64 / 128 and pages that are multiples of 16 only)."""
     T, Hq, D, num_pages, Hkv, page_size = _attn_common("attn_decode", q, k_pages, v_pages, out, q_start, kv_len,
@@ -1143,11 +1137,7 @@ def attn_decode(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, o
             float(scale), int(window), int(num_splits), sink.data_ptr(), status.data_ptr(), _stream())
         _done("attn_decode", code, f"heads {Hq}/{Hkv}, head_dim {D}, page {page_size}, with a sink")
         return
-    if beside and loader != "tma":
-        raise KernelError("attn_decode: only the kernel with the TMA loader runs beside another")
     fn = library().q3_attn_decode_tma if loader == "tma" else library().q3_attn_decode
-    if beside:
-        fn = library().q3_attn_decode_tma_beside
     code = fn(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(),
               _ptr(partial), q_start.data_ptr(), kv_len.data_ptr(), block_table.data_ptr(),
               block_table.shape[1], page_size, num_pages, num_seqs, Hq, Hkv, D, float(scale),
@@ -1281,14 +1271,6 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     if not fast_attention_takes(q.dtype, Hq, Hkv, D):
         attn_ref(q, k_pages, v_pages, out, q_start, kv_len, tok_seq, block_table, scale, window, status)
         return
-    tc = num_seqs > num_decode and portion_kernel != "mma" and attn_tc_takes(D, k_pages.shape[2], window)
-    if num_seqs > num_decode:
-        rest = (q_start[num_decode:], kv_len[num_decode:], block_table[num_decode:], num_seqs - num_decode, max_q_len)
-    if tc:
-        # ahead of the single tokens, which then run beside the portions: the places that short query tiles leave early
-        # are filled instead of waiting for the longest one (the other way round nothing overlaps: a portion's block
-        # needs a whole SM)
-        attn_tc(q, k_pages, v_pages, out, *rest, scale, status)
     if num_decode > 0:
         tma = decode_kernel != "cp_async" and decode_tma_takes(D, k_pages.shape[2])
         if tma:
@@ -1300,11 +1282,15 @@ def paged_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
         if partial is None or partial.numel() < num_decode * Hq * splits * (D + 2):
             splits = 1 if partial is None else max(1, partial.numel() // (num_decode * Hq * (D + 2)))
         attn_decode(q, k_pages, v_pages, out, partial, q_start, kv_len, block_table, num_decode, scale, window,
-                    splits, status, loader="tma" if tma else "cp_async", raw_qkv=raw_qkv, beside=tma and tc)
+                    splits, status, loader="tma" if tma else "cp_async", raw_qkv=raw_qkv)
     elif raw_qkv is not None:
         raise KernelError("paged_attention: the raw projection is only taken by a step of single tokens")
-    if num_seqs > num_decode and not tc:
-        attn_prefill(q, k_pages, v_pages, out, *rest, scale, window, status)
+    if num_seqs > num_decode:
+        rest = (q_start[num_decode:], kv_len[num_decode:], block_table[num_decode:], num_seqs - num_decode, max_q_len)
+        if portion_kernel != "mma" and attn_tc_takes(D, k_pages.shape[2], window):
+            attn_tc(q, k_pages, v_pages, out, *rest, scale, status)
+        else:
+            attn_prefill(q, k_pages, v_pages, out, *rest, scale, window, status)
 
 
 # ------------------------------------------------------------------ state carried from token to token

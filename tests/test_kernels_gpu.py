@@ -1069,44 +1069,6 @@ def run_fast(q, k_list, v_list, tables, num_pages, page_size, kv_lens, q_lens, w
     return torch.cat([pieces[i] for i in range(len(q_lens))])
 
 
-@pytest.mark.parametrize("d,hq,hkv,singles,portions", [
-    (128, 16, 8, [700, 65, 1, 333, 1500], [(37, 37), (900, 411)]),          # a few of each
-    (128, 16, 8, [40 + 29 * i for i in range(40)], [(600, 17)]),            # mostly single tokens
-    (64, 8, 2, [90], [(1200, 1200), (64, 2), (333, 200)]),                  # mostly portions, several per SM
-    (128, 32, 8, [16, 17], [(2500, 2300)])])
-def test_single_tokens_beside_portions(d, hq, hkv, singles, portions):
-    """A step with both: the single tokens' attention runs beside the portions', with the bits that each has alone, and what
-    is launched next finds both finished."""
-    o = ops()
-    kv_lens, q_lens = singles + [n for n, _ in portions], [1] * len(singles) + [m for _, m in portions]
-    q, k_list, v_list, tables, num_pages = attention_case("bfloat16", hq, hkv, d, 16, kv_lens, q_lens, None, seed=41)
-    k_pages, v_pages = (dev(paged(x, 16, tables, num_pages, torch.bfloat16)) for x in (k_list, v_list))
-    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))  # noqa: E731
-    starts = [sum(q_lens[:i]) for i in range(len(q_lens) + 1)]
-    n, Q, table, scale = len(singles), dev(q), dev(table_tensor(tables)), d ** -0.5
-    tok_seq = i32([b for b, m in enumerate(q_lens) for _ in range(m)])
-    partial = torch.empty(o.decode_partial_numel(len(q_lens), hq, d), device="cuda")
-    q_start, kv, st = i32(starts), i32(kv_lens), status()
-    alone = torch.full_like(Q, float("nan"))
-    splits = o.decode_splits(n, hkv, max(kv_lens), 0, d, blocks_per_sm=3, wide_blocks_per_sm=4)
-    o.attn_decode(Q, k_pages, v_pages, alone, partial, q_start, kv, table, n, scale, 0, splits, st, loader="tma")
-    torch.cuda.synchronize()
-    o.attn_tc(Q, k_pages, v_pages, alone, q_start[n:], kv[n:], table[n:], len(portions), max(q_lens), scale, st)
-    torch.cuda.synchronize()
-    weight = torch.ones(d, device="cuda")
-    want = torch.empty_like(Q)
-    o.rmsnorm(alone, weight, want, 1e-6)
-    for _ in range(5):
-        out, normed, fresh = torch.full_like(Q, float("nan")), torch.empty_like(Q), torch.zeros_like(Q)
-        partial.fill_(float("nan"))
-        o.rope(Q, torch.zeros(d // 2, device="cuda"), d, tok_seq, fresh, st)  # angles of zero: a copy, by a kernel of this library
-        o.paged_attention(fresh, k_pages, v_pages, out, q_start, kv, tok_seq, table, len(q_lens), n, max(q_lens), max(kv_lens),
-                          scale, 0, st, partial)
-        o.rmsnorm(out, weight, normed, 1e-6)
-        assert torch.equal(out, alone) and torch.equal(normed, want)
-    assert int(st.item()) == 0
-
-
 FAST_SHAPES = ATTN_SHAPES + [
     (16, 8, 128, 16, [700, 65, 1, 333], [1, 1, 1, 1], None),     # decode, the engine's big head size
     (16, 8, 128, 16, [700, 65, 130], [700, 64, 3], None),        # whole prompts and portions at head size 128
