@@ -27,6 +27,7 @@
 // Reference for the math: kernels/triton/paged_attn.py:89-181 (online softmax with exp2, P rounded
 // to the value dtype before P V), models/attn.py:388-400 (scale, causal on absolute positions).
 #include "tc_common.cuh"
+#include "tile_phase.h"
 
 namespace q3 {
 
@@ -83,10 +84,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   uint64_t* v_full = bars + 4;   // [2]
   uint64_t* v_empty = bars + 6;  // [2]
   uint64_t* s_ready = bars + 8;  // [2]
-  uint64_t* p_ready = bars + 10;
-  uint64_t* pv_done = bars + 11;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 12);
-  int* abort_word = reinterpret_cast<int*>(bars + 13);
+  uint64_t* p_ready = bars + 10;  // [2]
+  uint64_t* pv_done = bars + 12;  // [2]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 14);
+  int* abort_word = reinterpret_cast<int*>(bars + 15);
   float* row_xchg = reinterpret_cast<float*>(v_s + 2 * S::V_BYTES + S::BAR_BYTES);  // [2][parts][128] row maxima, then sums
 #define abort_flag (*abort_word)
 
@@ -128,9 +129,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       mbar_init(v_full + i, 1);
       mbar_init(v_empty + i, 1);
       mbar_init(s_ready + i, 1);
+      mbar_init(p_ready + i, AT_SOFTMAX / 32);
+      mbar_init(pv_done + i, 1);
     }
-    mbar_init(p_ready, AT_SOFTMAX / 32);
-    mbar_init(pv_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   pdl_wait();  // q and the pages come from the kernels before this one
@@ -202,7 +203,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     int page = page_id(0), page_next = page_id(1);
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
-      const int st = j & 1;
+      const int st = tile_slot(j);
       const uint32_t use = (uint32_t)j >> 1;
       const int page_after = page_id(j + 2);
       const bool wanted = has_page(j);
@@ -242,8 +243,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       const uint64_t k_desc0 = umma_desc_sw128(k_s), k_desc1 = umma_desc_sw128(k_s + S::K_BYTES);
       const uint64_t v_desc0 = umma_desc_sw128_mn(v_s, AT_BN * 128), v_desc1 = umma_desc_sw128_mn(v_s + S::V_BYTES, AT_BN * 128);
       auto issue_s = [&](int j) -> bool {
-        const int st = j & 1;
-        if (!mbar_wait(k_full + st, ((uint32_t)j >> 1) & 1, &abort_flag)) return false;
+        const int st = tile_slot(j);
+        if (!mbar_wait(k_full + st, tile_parity(j), &abort_flag)) return false;
         tcgen05_fence_after();
         const uint64_t kd = st ? k_desc1 : k_desc0;
         const uint32_t acc = tmem_s + st * AT_BN;
@@ -259,18 +260,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       };
       bool ok = issue_s(0);
       for (int j = 0; j < n_tiles && ok; ++j) {
-        const int st = j & 1;
+        const int st = tile_slot(j);
         if (j + 1 < n_tiles && !issue_s(j + 1)) { ok = false; break; }
-        if (!mbar_wait(p_ready, j & 1, &abort_flag)) { ok = false; break; }
-        if (!mbar_wait(v_full + st, ((uint32_t)j >> 1) & 1, &abort_flag)) { ok = false; break; }
+        if (!mbar_wait(p_ready + st, tile_parity(j), &abort_flag)) { ok = false; break; }
+        if (!mbar_wait(v_full + st, tile_parity(j), &abort_flag)) { ok = false; break; }
         tcgen05_fence_after();
         const uint64_t vd = st ? v_desc1 : v_desc0;
         const uint32_t p_cols = tmem_s + st * AT_BN;
 #pragma unroll
         for (int t = 0; t < AT_BN / 16; ++t)  // 16 keys: 8 packed columns of P, 16 rows (2048 bytes) of V
           umma_f16_ts(tmem_o, p_cols + 8 * t, vd + (uint64_t)(t * (2048 >> 4)), idesc_o, (j | t) != 0);
-        umma_commit(pv_done);
         umma_commit(v_empty + st);
+        umma_commit(pv_done + st);  // last: the last tile's is waited for, so no arrival is still to come when the block ends
       }
       if (!ok) {
         abort_flag = 1;
@@ -295,9 +296,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     // Every softmax thread runs every iteration and meets the others at the named barrier even
     // after a wait has run out (the barrier itself cannot time out); `ok` only switches the work off.
     for (int j = 0; j < n_tiles; ++j) {
-      const int st = j & 1;
+      const int st = tile_slot(j);
       float* xchg = row_xchg + (j & 1) * (AT_PARTS * AT_BM);
-      ok = ok && mbar_wait(s_ready + st, ((uint32_t)j >> 1) & 1, &abort_flag);
+      ok = ok && mbar_wait(s_ready + st, tile_parity(j), &abort_flag);
       tcgen05_fence_after();
       uint32_t sv[32];
       tmem_ld_32(tmem_s + st * AT_BN + part * AT_PART + lane_base, sv);
@@ -352,7 +353,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
       if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
         // O belongs to the tensor cores until the previous tile's P V has finished
-        ok = ok && mbar_wait(pv_done, (j - 1) & 1, &abort_flag);
+        ok = ok && mbar_wait(pv_done + tile_slot(j - 1), tile_parity(j - 1), &abort_flag);
         tcgen05_fence_after();
         // the row's threads rescale 32 output columns each (with D = 64 the first two of them)
         if (part * 32 < D) {
@@ -390,7 +391,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         }
       }
       if (tile_n + AT_BN > len) {
-        ok = ok && mbar_wait(v_full + st, ((uint32_t)j >> 1) & 1, &abort_flag);
+        ok = ok && mbar_wait(v_full + st, tile_parity(j), &abort_flag);
         const int first_bad = len - tile_n;
         for (int e = soft_tid; e < (AT_BN - first_bad) * (D / 8); e += AT_SOFTMAX) {
           const int key = first_bad + e / (D / 8), c = e % (D / 8);
@@ -403,18 +404,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       fence_async_proxy();
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_ready);
-      // SIGMOID never waits for a P V inside the loop to rescale; it follows them one tile behind here, where the
-      // product has had a whole tile's time to finish, so that the wait after the loop cannot mistake an earlier
-      // phase of the same parity for the last one
-      if (SIGMOID && j > 0) ok = ok && mbar_wait(pv_done, (j - 1) & 1, &abort_flag);
+      if (lane == 0) mbar_arrive(p_ready + st);
     }
     if (!ok && lane == 0) {
       abort_flag = 1;
       atomicOr(status, Q3_STATUS_TIMEOUT);
     }
     // the last P V, then O / l with l summed over the row's threads; each writes 32 of the columns
-    const bool done = ok && mbar_wait(pv_done, (n_tiles - 1) & 1, &abort_flag);
+    const bool done = ok && mbar_wait(pv_done + tile_slot(n_tiles - 1), tile_parity(n_tiles - 1), &abort_flag);
     float* xchg = row_xchg + (n_tiles & 1) * (AT_PARTS * AT_BM);
     xchg[part * AT_BM + rr] = l;
     asm volatile("bar.sync 1, %0;" ::"n"(AT_SOFTMAX) : "memory");
