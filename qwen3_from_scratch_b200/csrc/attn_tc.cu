@@ -202,6 +202,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     };
     int page = page_id(0), page_next = page_id(1);
     bool ok = true;
+    uint32_t issued = 0;  // tiles asked for
     for (int j = 0; j < n_tiles; ++j) {
       const int st = tile_slot(j);
       const uint32_t use = (uint32_t)j >> 1;
@@ -223,6 +224,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         for (int a = 0; a < ATOMS; ++a)
           tma_load_2d(dst_base + st * S::K_BYTES + a * (AT_BN * 128) + lane * page_size * 128, map, full + st, a * 64, y);
       }
+      if (ok) ++issued;
       page = page_next;
       page_next = page_after;
     }
@@ -230,6 +232,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       abort_flag = 1;
       atomicOr(status, Q3_STATUS_TIMEOUT);
     }
+    if (lane == 0) finish_copies(full, issued, 2, is_v ? -1 : tc_drop_copy, status);
   } else if (warp == AT_ISSUE_WARP) {
     // ------------------------------------------------------------------ tensor-core issue
     if (lane == 0) {

@@ -492,6 +492,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           tma_load_2d(a_s, &map_a, &full[s], kt * TC_BK, m0);
         }
       }
+      finish_copies(full, it, S::STAGES, tc_drop_copy, status);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -709,6 +710,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           tma_load_2d_pair(a_s, &map_a, pair_full, kt * TC_BK, m0);
         }
       }
+      if (rank == 0) finish_copies(full, it, S::STAGES, tc_drop_copy, status);  // its barriers count both CTAs' copies
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {

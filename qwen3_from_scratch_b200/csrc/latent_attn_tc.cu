@@ -176,7 +176,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_c
       uint64_t* full = is_v ? v_full : k_full;
       uint64_t* empty = is_v ? v_empty : k_empty;
       bool ok = true;
-      int last = -1;  // the last tile asked for
+      uint32_t issued = 0;  // tiles asked for
       for (int j = 0; j < n_tiles && ok; ++j) {
         const int st = tile_slot(j), y = b * pitch + j * LT_BN;
         if (j > 1) ok = mbar_wait(empty + st, ((uint32_t)(j >> 1) - 1) & 1, &abort_flag);
@@ -191,18 +191,13 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_c
             tma_load_2d(k_s + st * LT_K_BYTES + a * LT_ATOM, &map_kv, full + st, h * LT_D + a * 64, y);
           tma_load_2d(k_s + st * LT_K_BYTES + (LT_D / 64) * LT_ATOM, &map_r, full + st, 0, y);
         }
-        last = j;
+        ++issued;
       }
       if (!ok) {
         abort_flag = 1;
         atomicOr(status, Q3_STATUS_TIMEOUT);
       }
-      // A block that gives up may not have consumed its last two copies: it must not leave while they are on their way into
-      // its shared memory.  (Otherwise they are long complete.)  The flag above does not cut these waits short.
-      int never = 0;
-      for (int j = max(0, last - 1); j <= last; ++j)
-        if ((is_v || j != tc_drop_copy) && !mbar_wait(full + (j & 1), ((uint32_t)j >> 1) & 1, &never))
-          atomicOr(status, Q3_STATUS_TIMEOUT);
+      finish_copies(full, issued, 2, is_v ? -1 : tc_drop_copy, status);
     }
   } else if (warp == LT_ISSUE_WARP) {
     // ------------------------------------------------------------------ tensor-core issue

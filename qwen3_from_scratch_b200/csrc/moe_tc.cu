@@ -274,6 +274,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           tma_load_2d(a_s, &map_a, &full[s], kt * TC_BK, m0);
         }
       }
+      finish_copies(full, it, S::STAGES, -1, status);
     }
   } else if (warp == 1) {
     if (lane == 0) {

@@ -70,6 +70,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// What a loader does last: copy u of its `issued` copies went to stage u % stages, whose `full` barrier counts it.  A block
+// that gives up may not have consumed its last round of copies, and must not leave while they are on their way into its
+// shared memory.  (Otherwise they are long complete.)  The abort flag does not cut these waits short; once one has run out,
+// the others' time is over too.  `dropped`: the copy that the tests leave out, or -1.
+__device__ __forceinline__ void finish_copies(uint64_t* full, uint32_t issued, uint32_t stages, int dropped, int* status) {
+  int never = 0;
+  for (uint32_t u = issued > stages ? issued - stages : 0; u < issued; ++u)
+    if ((int)u != dropped && !mbar_wait(full + u % stages, (u / stages) & 1, &never)) {
+      atomicOr(status, Q3_STATUS_TIMEOUT);
+      return;
+    }
+}
+
 // Brings a tensor map into the descriptor cache ahead of its first use by a copy.
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
