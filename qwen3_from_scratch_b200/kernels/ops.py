@@ -1031,14 +1031,14 @@ DECODE_LONG_BLOCK = (0.15, 128)  # a single wave of that form: per tile of a blo
 
 
 def decode_splits(num_seqs: int, num_kv_heads: int, max_kv_len: int, window: int, head_dim: int = 128,
-                  blocks_per_sm: Optional[int] = None, wide_blocks_per_sm: Optional[int] = None) -> int:
+                  blocks_per_sm: Optional[int] = None, wide_blocks_per_sm: Optional[int] = None, merge_tiles: float = 0) -> int:
     """How many ranges a sequence's keys are cut into.  Blocks run in waves of (SMs x blocks per SM).  A
     block alone walks its 16-key tiles at its own pace; ``DECODE_SATURATING`` blocks per SM together take
     tiles as fast as the memory gives them, and more blocks then only share that rate; every wave after the
     first costs a start.  So a wave of n blocks of L tiles costs max(L, n L / saturating), and the count with
     the least sum over its waves wins, the smaller count on a tie.  ``wide_blocks_per_sm``: the kernel has a
     form with that many (smaller) blocks per SM, which the launcher takes for a grid that ``blocks_per_sm``
-    do not hold at once.  The constants are fitted to sweeps of the decode step over batch and context
+    do not hold at once.  ``merge_tiles``: what more than one range costs beside that, in tiles.  The constants are fitted to sweeps of the decode step over batch and context
     (profiles/attn_decode_tma__decode_b8_ctx4096.md)."""
     span = min(max_kv_len, window) if window and window > 0 else max_kv_len
     tiles = max(1, -(-span // 16))
@@ -1063,6 +1063,8 @@ def decode_splits(num_seqs: int, num_kv_heads: int, max_kv_len: int, window: int
             cost += DECODE_WIDE_GRID
             if waves == 1:
                 cost += DECODE_LONG_BLOCK[0] * max(0, per_block - DECODE_LONG_BLOCK[1])
+        if s > 1:
+            cost += merge_tiles
         if best_cost is None or cost < best_cost - 1e-6:
             best, best_cost = s, cost
     return best
@@ -1552,6 +1554,19 @@ def sigmoid_decode_splits(num_seqs: int, num_kv_heads: int, max_kv_len: int) -> 
     return max(1, min(SIGMOID_MAX_SPLITS, tiles // 4, want))
 
 
+SIGMOID_SUM_TILES = 10  # what the launch that adds the ranges up costs, in tiles of a block
+
+
+def sigmoid_tma_decode_splits(num_seqs: int, num_kv_heads: int, max_kv_len: int, head_dim: int) -> int:
+    """Key ranges of the decode form with the TMA loader: ``decode_splits`` for the softmax form of the same kernel, with the
+    sum's launch (1.5 to 2 us, 0.2 to 0.3 us a tile) and its reading charged.  Measured over batch, context and heads against the
+    cp.async kernel under its own rule: without the charge up to 11 % slower at 130 to 256 keys (16 query heads over 2 of 64, batch
+    64, 130 keys: two ranges 5.7 us, the cp.async kernel 5.1, one range 4.0), with 6 tiles up to 6 % (16 over 1 of 128, batch 128, 200
+    keys: 11.2 and 10.5), with 10 nowhere; beyond 300 keys 1.04 to 3.7 times faster with any of them."""
+    return decode_splits(num_seqs, num_kv_heads, max_kv_len, 0, head_dim, blocks_per_sm=3, wide_blocks_per_sm=4,
+                         merge_tiles=SIGMOID_SUM_TILES)
+
+
 def attn_sigmoid_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor,
                      head_bias: Optional[torch.Tensor], gate: Optional[torch.Tensor], q_start: torch.Tensor,
                      kv_len: torch.Tensor, block_table: torch.Tensor, num_seqs: int, max_q_len: int, scale: float,
@@ -1634,9 +1649,9 @@ def sigmoid_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         return
     decode = num_decode if Hq // Hkv <= 16 else 0  # a wider group's single tokens run as portions of one
     if decode > 0:
-        # the TMA loader where it takes the shape, with the ranges of the softmax's decode kernel (the same blocks and bytes)
+        # the TMA loader where it takes the shape
         tma = kernel != "mma" and decode_tma_takes(D, k_pages.shape[2])
-        splits = (decode_splits(decode, Hkv, max_kv_len, 0, D, blocks_per_sm=3, wide_blocks_per_sm=4) if tma
+        splits = (sigmoid_tma_decode_splits(decode, Hkv, max_kv_len, D) if tma
                   else sigmoid_decode_splits(decode, Hkv, max_kv_len))
         if partial is None or partial.numel() < decode * splits * Hq * D:
             splits = 1 if partial is None else max(1, partial.numel() // (decode * Hq * D))

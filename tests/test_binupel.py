@@ -135,3 +135,19 @@ def test_plain_mechanisms_on_values_worked_by_hand():
     tau = plain.query_temperature(torch.tensor([0, 5, 6, 13]), 1.0, 7)
     assert torch.allclose(tau, 1 + torch.log(torch.tensor([1.0, 1.0, 2.0, 3.0], dtype=plain.F64)))
     assert abs(float(plain.gelu_tanh(torch.tensor(1.0, dtype=plain.F64))) - 0.8411919906082768) < 1e-12
+
+
+def test_key_ranges_of_sigmoid_decoding(monkeypatch):
+    """A context that a block walks in less time than the sum of ranges takes to launch stays in one range; a long one of a
+    small batch is cut, never into ranges of fewer than four tiles, and the softmax form's rule is what it was."""
+    from qwen3_from_scratch_b200.kernels import ops
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    for batch in (1, 4, 16, 64, 128):
+        for kv_heads in (1, 2, 8):
+            for keys in (1, 16, 64, 130, 160):
+                assert ops.sigmoid_tma_decode_splits(batch, kv_heads, keys, 128) == 1
+    softmax = dict(blocks_per_sm=3, wide_blocks_per_sm=4)
+    assert ops.decode_splits(16, 8, 130, 0, 128, **softmax) == 2
+    for batch, keys in ((1, 517), (8, 2048), (16, 1024), (2, 8192)):
+        ranges = ops.sigmoid_tma_decode_splits(batch, 8, keys, 128)
+        assert 1 < ranges == ops.decode_splits(batch, 8, keys, 0, 128, **softmax) and -(-keys // 16) // ranges >= 4
