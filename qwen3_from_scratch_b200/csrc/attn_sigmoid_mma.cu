@@ -240,7 +240,7 @@ sum_gate_kernel(const float* __restrict__ partial, const float* __restrict__ gat
                 __nv_bfloat16* __restrict__ out, int Hq, int D, int num_splits) {
   pdl_wait();
   pdl_launch_dependents();
-  const int b = blockIdx.x, row = Hq * D, e = (blockIdx.y * SG_THREADS + threadIdx.x) * 2;  // D is even
+  const int b = blockIdx.y, row = Hq * D, e = (blockIdx.x * SG_THREADS + threadIdx.x) * 2;  // D is even
   if (e >= row) return;
   const int t = q_start[b];
   const float gt = gate ? gate[(size_t)t * Hq + e / D] : 1.f;
@@ -285,12 +285,11 @@ static int attn_sigmoid_mma_launch(const void* q, const void* k_pages, const voi
 
 }  // namespace q3
 
-// The sum of the key ranges, for every decode kernel that leaves partial sums [B, num_splits, Hq, D] (D even).
+// The sum of the key ranges, for every decode kernel that leaves partial sums [B, num_splits, Hq, D] (D even, B up to 65,535).
 extern "C" int q3_sum_gate(const float* partial, const float* gate, const int* q_start, void* out, int B, int Hq, int D,
                            int num_splits, cudaStream_t stream) {
-  const int pieces = (Hq * D / 2 + q3::SG_THREADS - 1) / q3::SG_THREADS;
-  if (pieces > 65535) return Q3_ERR_SIZE;
-  q3::launch(q3::sum_gate_kernel, dim3(B, pieces), dim3(q3::SG_THREADS), 0, stream, partial, gate, q_start, (__nv_bfloat16*)out,
+  const unsigned pieces = (unsigned)((Hq * D / 2 + q3::SG_THREADS - 1) / q3::SG_THREADS);
+  q3::launch(q3::sum_gate_kernel, dim3(pieces, B), dim3(q3::SG_THREADS), 0, stream, partial, gate, q_start, (__nv_bfloat16*)out,
              Hq, D, num_splits);
   return q3::launch_status();
 }

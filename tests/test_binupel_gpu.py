@@ -373,6 +373,31 @@ def test_single_tokens_with_sigmoid_weights_by_the_tma_loader(hq, hkv, d, page, 
         assert float((got.float() - want.float()).abs().max()) <= 1.5e-2 * float(want.float().abs().max())
 
 
+@pytest.mark.parametrize("loader", ["cp_async", "tma"])
+def test_the_sum_of_key_ranges_takes_as_many_heads_as_the_attention(loader):
+    """131,072 heads of 128 (more than 65,535 pieces of 256 values for one request), two ranges of 16 keys.  Each weight
+    w_n and the result are rounded to bfloat16 once, by up to 2^-8 of themselves: no value is further off than
+    2^-8 (sum_n w_n |v_n| + |result|), and a little for the sums' own roundings."""
+    from qwen3_from_scratch_b200.kernels import ops
+    hkv, group, d, n = 8192, 16, 128, 32
+    g = torch.Generator(device="cuda").manual_seed(47)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    k_pages, v_pages, q = rand(2, hkv, 16, d), rand(2, hkv, 16, d), rand(1, hkv * group, d)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    status, out = i32([0]), torch.full_like(q, float("nan"))
+    partial = torch.full((2 * q.numel(),), float("nan"), device="cuda")
+    ops.attn_sigmoid_mma(q, k_pages, v_pages, out, None, None, i32([0, 1]), i32([n]), i32([[1, 0]]), 1, 1, d ** -0.5, status,
+                         decode=True, num_splits=2, partial=partial, loader=loader)
+    assert int(status.item()) == 0
+    for h in range(0, hkv, 1024):
+        k, v = (torch.cat((p[1, h:h + 1024], p[0, h:h + 1024]), dim=1).double() for p in (k_pages, v_pages))
+        weights = torch.sigmoid(q.view(hkv, group, d)[h:h + 1024].double() @ k.transpose(1, 2) * d ** -0.5)
+        want = weights @ v
+        got = out.view(hkv, group, d)[h:h + 1024].double()
+        worst = float(((got - want).abs() / (weights @ v.abs() + want.abs())).max())
+        assert worst <= 1.01 * 2.0 ** -8, worst
+
+
 # ---------------------------------------------------------------------- whole models
 def tolerance(dtype, cfg, w, seqs):
     """float32: the harness's bound.  bfloat16: three times what rounding alone does to these prompts in the plain
