@@ -501,10 +501,9 @@ extern "C" int q3_attn_combine(const float* partial, void* out, const int* q_sta
   if (B <= 0 || num_splits <= 1) return 0;
   if (D <= 0 || D > q3::AC_MAX_D || (D & 1)) return Q3_ERR_SIZE;
   dim3 cgrid(Hq, B);
-  // The merge starts when the attention has completed, not early (the one ordinary launch of a decode step):
-  // its blocks, resident and waiting while the attention still has blocks to place, took the places of those
-  // blocks.  With 256 merge blocks beside a grid of two waves (the 8B sizes, batch 8 at a context of 16,384)
-  // the attention ran twice as long and the step 28 % longer.
+  // The merge starts when the attention has completed, not early (the one ordinary launch of a decode step).  Launched
+  // early, 256 merge blocks beside a grid of two waves (the 8B sizes, batch 8 at a context of 16,384) made the attention
+  // twice and the step 28 % longer: its blocks, resident and waiting, hold places that the attention's last blocks need.
   q3::g_launch_early = false;
   q3::launch(q3::attn_combine_kernel, cgrid, dim3(q3::AC_WARPS * 32), 0, stream, partial, (__nv_bfloat16*)out, q_start, Hq, D,
              num_splits);

@@ -7,11 +7,11 @@
 // a bandwidth-bound kernel wants, and the consumers issue no copy instructions at all.
 //
 // SIGMOID: the weights of attn_sigmoid.cu (sigmoid(s * scale + head_bias[h]), not normalised; the finished row times
-// gate[t, h]): no maximum, no denominator, and the ranges' partial sums are plain sums.  (Eight requests at 2,048 tokens, 16 heads over 8 of
-// 128, inside a step: 16 us where the cp.async kernel took 29, for 10 of cache bytes.)
+// gate[t, h]): no maximum, no denominator, and the ranges' partial sums are plain sums.  (Eight requests at 2,048 tokens,
+// 16 heads over 8 of 128, inside a step: 16 us where the cp.async kernel took 29, for 10 of cache bytes.)
 //
-// Takes D = 64 or 128 and page sizes that are multiples of 16 (a 16-key tile then lies in one
-// page); everything else goes to attn_decode.cu.  Mbarrier waits are bounded (tc_common.cuh).
+// Takes D = 64 or 128 and page sizes that are multiples of 16 (a 16-key tile then lies in one page); everything else goes to
+// attn_decode.cu, and with sigmoid weights to attn_sigmoid_mma.cu.  Mbarrier waits are bounded (tc_common.cuh).
 #include "attn_mma.cuh"
 #include "tc_common.cuh"
 
@@ -120,8 +120,8 @@ struct DecodeQkv {
 // BLOCKS: blocks per SM the kernel is compiled for.  Three (128 registers) give a large grid half as many
 // places again as two; two (168 registers) are the faster code where the grid fits their places anyway; four
 // (smaller blocks, see DecodeTmaBlock) are for a grid of several waves, where more blocks per SM in different
-// stages of their lives keep the SM's stream over the cache going
-// (figures: profiles/attn_decode_tma__decode_b8_ctx4096.md).
+// stages of their lives keep the SM's stream over the cache going (kernel and merge, batch 64, 32/8 heads, three and four blocks:
+// 79 and 66 us at a context of 1,280, 184 and 169 at 4,096).
 template <int D, int BLOCKS, bool SIGMOID = false>
 __global__ void __launch_bounds__(DecodeTmaBlock<BLOCKS>::THREADS, BLOCKS)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -377,41 +377,41 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           }
       }
       if (!SIGMOID) {
-      float mx[2];
-      mx[0] = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
-      mx[1] = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
-      float alpha[2], m_use[2];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-        const float m_new = fmaxf(m[r], mx[r] * scale_log2);
-        m_use[r] = m_new == -INFINITY ? 0.f : m_new;
-        alpha[r] = exp2f(m[r] - m_use[r]);
-        m[r] = m_new;
-      }
-      if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
+        float mx[2];
+        mx[0] = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
+        mx[1] = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
+        float alpha[2], m_use[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          l[r] *= alpha[r];
+          mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+          mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+          const float m_new = fmaxf(m[r], mx[r] * scale_log2);
+          m_use[r] = m_new == -INFINITY ? 0.f : m_new;
+          alpha[r] = exp2f(m[r] - m_use[r]);
+          m[r] = m_new;
+        }
+        if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
 #pragma unroll
-          for (int i2 = 0; i2 < 2 * KT; ++i2) {
-            o[i2][2 * r] *= alpha[r];
-            o[i2][2 * r + 1] *= alpha[r];
+          for (int r = 0; r < 2; ++r) {
+            l[r] *= alpha[r];
+#pragma unroll
+            for (int i2 = 0; i2 < 2 * KT; ++i2) {
+              o[i2][2 * r] *= alpha[r];
+              o[i2][2 * r + 1] *= alpha[r];
+            }
           }
         }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            const float p0 = exp2f(fmaf(sc[nt][2 * r], scale_log2, -m_use[r]));
+            const float p1 = exp2f(fmaf(sc[nt][2 * r + 1], scale_log2, -m_use[r]));
+            sc[nt][2 * r] = p0;
+            sc[nt][2 * r + 1] = p1;
+            l[r] += p0 + p1;
+          }
       }
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const float p0 = exp2f(fmaf(sc[nt][2 * r], scale_log2, -m_use[r]));
-          const float p1 = exp2f(fmaf(sc[nt][2 * r + 1], scale_log2, -m_use[r]));
-          sc[nt][2 * r] = p0;
-          sc[nt][2 * r + 1] = p1;
-          l[r] += p0 + p1;
-        }
-      }  // softmax
       uint32_t pa[4];
       pa[0] = pack_bf16(sc[0][0], sc[0][1]);
       pa[1] = pack_bf16(sc[0][2], sc[0][3]);
@@ -530,9 +530,10 @@ static int attn_decode_tma_launch(const void* q, const void* k_pages, const void
   // two blocks per SM where the grid fits them, three where it fits those, four for a grid of several waves
   const int per_sm = blocks <= 2LL * sm_count() ? 2 : blocks <= 3LL * sm_count() ? 3 : 4;
 #define Q3_DT_LAUNCH(BL)                                                                                              \
-  q3::launch(attn_decode_tma_kernel<D, BL, SIGMOID>, grid, dim3(DecodeTmaBlock<BL>::THREADS), DecodeTmaShape<D, BL>::SMEM_BYTES,  \
-             stream, map_k, map_v, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, partial, q_start, kv_len, block_table, \
-             table_stride, page_size, num_pages, Hq, Hkv, scale * 1.4426950408889634f, window, num_splits, status, fq)
+  q3::launch(attn_decode_tma_kernel<D, BL, SIGMOID>, grid, dim3(DecodeTmaBlock<BL>::THREADS),                         \
+             DecodeTmaShape<D, BL>::SMEM_BYTES, stream, map_k, map_v, (const __nv_bfloat16*)q, (__nv_bfloat16*)out,   \
+             partial, q_start, kv_len, block_table, table_stride, page_size, num_pages, Hq, Hkv,                      \
+             scale * 1.4426950408889634f, window, num_splits, status, fq)
   if (per_sm == 2) Q3_DT_LAUNCH(2);
   else if (per_sm == 3) Q3_DT_LAUNCH(3);
   else Q3_DT_LAUNCH(4);

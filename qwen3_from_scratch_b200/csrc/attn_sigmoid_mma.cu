@@ -232,8 +232,10 @@ attn_sigmoid_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 }
 
 // out[t(b), h, :] = gate * sum over the key ranges of partial[b, s, h, :], ranges in ascending order.  Two values per thread
-// and all ranges' loads in flight (four at a time): with a block per request, 256 threads and one load after the other
-// eight requests of 16 heads of 128 took 6 us behind the attention, now under 3.
+// and four ranges' loads in flight: with a block per request, 256 threads and one load after the other eight requests of 16 heads
+// of 128 took 6 us behind the attention, now under 3.  Launched early, unlike the softmax's merge (attn_decode.cu): over 468 points
+// of batch, context and heads behind the TMA kernel an ordinary launch was slower by more than 3 % at 237 (up to 4 us) and faster
+// at 11 (16 query heads over one kv head, batch 16 and 32: up to 11 %).
 constexpr int SG_THREADS = 128;
 __global__ void __launch_bounds__(SG_THREADS)
 sum_gate_kernel(const float* __restrict__ partial, const float* __restrict__ gate, const int* __restrict__ q_start,

@@ -24,8 +24,10 @@ constexpr int GF_LANE = 8;    // values of k of a lane at a time
 // and the four partial sums meet in shared memory (64 FMA per four 16-byte shared-memory reads).  The split over K inside
 // the block gives a narrow product more blocks than wider tiles would (N = 1,024 and 500 rows: 128 tiles of 64 x 64, with
 // eight warps each, against 32 of 128 x 128 for 148 SMs).  The FMA pipe is busy half of the time (513 x 4,096 x 1,024: 139.8 us,
-// 31 of 74 TFLOP/s): register-bank conflicts of 128 accumulators and the start of each tile, which nothing covers with one
-// block per SM, take the rest.
+// 31 of 74 TFLOP/s).  Of 5.4 us for a tile's 128 values of k the FMA loop alone takes 3.2 (49 TFLOP/s; such a loop over registers
+// reaches 50 to 72, by how the compiler places them), and two warps per scheduler hide none of the rest: operand reads 1.2,
+// copies 0.6, running sums 0.6.  Packed FMAs reach 61 to 73 in such a loop, and 0.8 to 1.0 of this kernel's speed in it where the
+// tiles fill the SMs.
 constexpr int GF_T = 64, GF_GROUPS = 4, GF_GROUP_THREADS = 64, GF_THREADS = GF_GROUPS * GF_GROUP_THREADS, GF_STAGES = 3;
 constexpr int GF_STAGE_BYTES = 2 * GF_T * 128;                            // 64 rows of A, 64 of W, 32 values of k each
 constexpr int GF_RED_PITCH = GF_T + 8;                                    // floats: a thread's rows fall on different banks

@@ -54,8 +54,8 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 // stream of the output head, and with two token tiles: there, left to itself, the compiler used fewer registers
 // than three blocks allow and took the loads one after the other.  Two token tiles are short of registers at
 // three blocks per SM, though: where the grid fits two blocks per SM (ROOMY) the kernel is asked for two.  A warp
-// that fetches two or three batches ahead gets all the registers it wants.  Figures:
-// profiles/gemm_skinny__decode_b8.md.)
+// that fetches two or three batches ahead gets all the registers it wants.  16 rows into a stream of 4,096 features from 12,288
+// inputs: 33.9 us at three blocks, 22.5 at two; the output head's 311 MB at 6.1 TB/s.)
 // PRE: batches of GS_UNROLL groups whose weights are fetched before the wait on the kernel before.  A
 // product with few output features (o_proj, down_proj: 64 groups of 16, one block each) gives a warp two or
 // three batches; with all of them under way before the wait, what is left after it is one round trip for

@@ -36,13 +36,6 @@ __device__ __forceinline__ void split_bf16x4(float4 v, uint2& hi, uint2& lo) {
   hi = make_uint2(pack_bf16(__bfloat162float(h[0]), __bfloat162float(h[1])), pack_bf16(__bfloat162float(h[2]), __bfloat162float(h[3])));
   lo = make_uint2(pack_bf16(__bfloat162float(l[0]), __bfloat162float(l[1])), pack_bf16(__bfloat162float(l[2]), __bfloat162float(l[3])));
 }
-// 16 bytes into shared memory, or zeros.
-__device__ __forceinline__ void sm_copy16(void* dst, const void* src, bool in) {
-  const int n = in ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n)
-               : "memory");
-}
-
 // What both kernels do first: the chunk's rows of x (this head's P channels), B and C (its group's N values) into
 // shared memory as [SM_Q][P + 8] and [SM_Q][N + 8], zero beyond the chunk's end; step sizes and the inclusive sums of
 // the log-decays (a row beyond the end has step 0 and decay 1: it changes nothing).
@@ -56,15 +49,15 @@ __device__ __forceinline__ void load_chunk(const __nv_bfloat16* __restrict__ xbc
   const __nv_bfloat16* const rows = xbc + (size_t)t0 * ld;
   for (int i = threadIdx.x; i < SM_Q * (P / 8); i += blockDim.x) {
     const int t = i / (P / 8), c = i % (P / 8);
-    sm_copy16(xs + t * PX + c * 8, rows + (t < len ? (size_t)t * ld + h * P + c * 8 : 0), t < len);
+    cp_async_16(xs + t * PX + c * 8, rows + (t < len ? (size_t)t * ld + h * P + c * 8 : 0), t < len ? 16 : 0);
   }
   for (int i = threadIdx.x; i < SM_Q * (N / 8); i += blockDim.x) {
     const int t = i / (N / 8), c = i % (N / 8);
     const __nv_bfloat16* row = rows + (t < len ? (size_t)t * ld + inner + g * N + c * 8 : 0);
-    sm_copy16(bs + t * PN + c * 8, row, t < len);
-    if (WANT_C) sm_copy16(cs + t * PN + c * 8, row + (t < len ? (size_t)G * N : 0), t < len);
+    cp_async_16(bs + t * PN + c * 8, row, t < len ? 16 : 0);
+    if (WANT_C) cp_async_16(cs + t * PN + c * 8, row + (t < len ? (size_t)G * N : 0), t < len ? 16 : 0);
   }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+  cp_async_commit();
   if (threadIdx.x < SM_Q) {
     const int t = threadIdx.x;
     float step = 0.f;
@@ -97,7 +90,7 @@ __device__ __forceinline__ void load_chunk(const __nv_bfloat16* __restrict__ xbc
       }
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  cp_async_wait<0>();
   __syncthreads();
 }
 
@@ -232,8 +225,9 @@ ssd_chunk_carry_kernel(float* __restrict__ scratch, float* __restrict__ state, c
 // grid (requests, chunks, heads), 128 threads: warp w owns the chunk's rows 16 w .. 16 w + 15.
 // A block is a chain of latencies (rows, decays, products, state, products), so as many as possible share an SM: the state
 // takes the place of B and C once their product is in registers (47 KB, four blocks; two while each had its own), and is
-// asked into L2 before the block waits for anything.  (32 chunks of 64 heads of 64 x 128 inside a step: 87 us before, 59 now, for
-// 115 MB; the states' kernel, whose weighted x is split eight values at a time, 39 and 30.)
+// asked into L2 before the block waits for anything.  (32 chunks of 64 heads of 64 x 128, 115 MB, one launch at a time with
+// cold caches: 52 us, 79 before; the states' kernel, whose weighted x is split eight values at a time, 32 and 41; the three
+// launches replayed one behind the other 104 and 139 a call.)
 template <int P, int N>
 __global__ void __launch_bounds__(128, 4)
 ssd_chunk_output_kernel(const __nv_bfloat16* __restrict__ xbc, int ld, const __nv_bfloat16* __restrict__ proj, int ld_proj,
