@@ -146,13 +146,14 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int gid = lane >> 2, tid4 = lane & 3;
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int g = Hq / Hkv;
+  const bool raw = !SIGMOID && fq.qkv != nullptr;  // the sigmoid form has no raw projection, no sink and no window
   const int tq = q_start[b];
   const int pos = kv_len[b] - 1;
   const int* table = block_table + (size_t)b * table_stride;
 
   int t_lo = 0, t_hi = 0, lo = 0;
   if (pos >= 0) {
-    lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+    lo = (!SIGMOID && window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
     const int first = lo / DT_KEYS, last = pos / DT_KEYS;
     const int per = (last - first + num_splits) / num_splits;
     t_lo = first + split * per;
@@ -181,7 +182,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   // one (which writes this step's key, value and query) may still be running.  Only the tile that
   // holds the sequence's last position, and the query, wait for that kernel.
   if (warp != DT_CONSUMERS) {
-    if (fq.qkv != nullptr) {
+    if (raw) {
       // the norm weights, which no kernel writes, and the token's cosines and sines, if the launch before this
       // one did not write them, are asked into L1 ahead of the wait (D floats each: D / 32 lines of 128 bytes)
       constexpr int LINES = D / 32;
@@ -195,7 +196,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     for (int e = threadIdx.x; e < 16 * CPR; e += DT_CONSUMERS * 32) {
       const int row = e / CPR, c = e % CPR;  // a row's CPR chunks of eight values sit in neighbouring lanes
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (fq.qkv == nullptr) {
+      if (!raw) {
         if (row < g) v = *reinterpret_cast<const uint4*>(q + ((size_t)tq * Hq + hk * g + row) * D + c * 8);
       } else {
         // the raw projection's head hk * g + row: head norm, then rotation (every lane takes part in the shuffles)
@@ -282,7 +283,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       unsigned char* v_t = ring + (size_t)s * S::STAGE_BYTES + S::TILE_BYTES;
       const int base_n = (t_lo + i) * DT_KEYS;
       const bool edge = base_n < lo || base_n + DT_KEYS - 1 > pos;
-      if (fq.qkv != nullptr && fq.write_kv && t_lo + i == pos / DT_KEYS) {
+      if (raw && fq.write_kv && t_lo + i == pos / DT_KEYS) {
         // this step's key and value: made here from the raw projection, written to their page for the steps
         // to come and into this tile, which was fetched without them.  A lane holds D / 32 neighbouring values.
         constexpr int VPL = D / 32;
@@ -477,7 +478,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
     }
     const int head = hk * g + r;
-    if (fq.sink != nullptr && split == 0) {  // the sink: one more exponential in the denominator, in the first range's share
+    if (!SIGMOID && fq.sink != nullptr && split == 0) {  // the sink: one more exponential in the denominator, in the first range's share
       const float s2 = fq.sink[head] * 1.4426950408889634f, top = fmaxf(big, s2);
       const float keep = big == -INFINITY ? 0.f : exp2f(big - top);
       acc *= keep;
